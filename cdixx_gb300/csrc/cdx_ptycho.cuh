@@ -114,7 +114,8 @@ template <int N>
 struct PtyRow {
   static constexpr int SN = N + 8;
   static constexpr int STAGE = 2 * Geom<N>::L * SN * (int)sizeof(float2);
-  static constexpr int SMEM = Geom<N>::SMEM_LINES + STAGE;
+  static constexpr int LD = RGeom<N>::ROW_LD;
+  static constexpr int SMEM = RGeom<N>::SMEM_ROW_LINES + STAGE;
 };
 
 template <int N>
@@ -143,14 +144,14 @@ __global__ void __launch_bounds__(Geom<N>::T, Geom<N>::MINB) pty_fwd_rk(PtyArgs 
   constexpr int L = G::L;
   using F0 = RFirst<N, 0>;
   using FL = RLast<N, 0>;
-  constexpr int SN = PtyRow<N>::SN;
+  constexpr int SN = PtyRow<N>::SN, LD = PtyRow<N>::LD;
   extern __shared__ float2 smem[];
   pdl_wait_and_release();
-  float2* o_s = smem + L * G::LD;
+  float2* o_s = smem + L * LD;
   float2* p_s = o_s + L * SN;
   const int row0 = blockIdx.x * L;
   const int nrows = min(L, a.rows - row0);
-  const int cb = min(a.tl, rfft_cb_max<N>());
+  const int cb = row_cb_pick(a.tl, rfft_cb_max<N>());
   const int si = a.order[*a.iter * a.nscan + a.k];
   pty_stage_rows<N>(a, o_s, p_s, row0, nrows, a.win[si]);
   cp_wait<0>();
@@ -168,7 +169,7 @@ __global__ void __launch_bounds__(Geom<N>::T, Geom<N>::MINB) pty_fwd_rk(PtyArgs 
     }
   }
   float2 v[FL::B][FL::R];
-  rfft<N, 0, false>(v0, v, smem, a.tw, cb);
+  rfft<N, 0, false, LD>(v0, v, smem, a.tw, cb);
 #pragma unroll
   for (int b = 0; b < FL::B; ++b) {
     int l, j;
@@ -260,14 +261,14 @@ __global__ void __launch_bounds__(Geom<N>::T, Geom<N>::MINB) pty_upd_rk(PtyArgs 
   constexpr int L = G::L;
   using F0 = RFirst<N, 0>;
   using FL = RLast<N, 0>;
-  constexpr int SN = PtyRow<N>::SN;
+  constexpr int SN = PtyRow<N>::SN, LD = PtyRow<N>::LD;
   extern __shared__ float2 smem[];
   pdl_wait_and_release();
-  float2* o_s = smem + L * G::LD;
+  float2* o_s = smem + L * LD;
   float2* p_s = o_s + L * SN;
   const int row0 = blockIdx.x * L;
   const int nrows = min(L, a.rows - row0);
-  const int cb = min(a.tl, rfft_cb_max<N>());
+  const int cb = row_cb_pick(a.tl, rfft_cb_max<N>());
   const int si = a.order[*a.iter * a.nscan + a.k];
   const int2 w = a.win[si];
   const long long OC = a.obj_cols;
@@ -282,7 +283,7 @@ __global__ void __launch_bounds__(Geom<N>::T, Geom<N>::MINB) pty_upd_rk(PtyArgs 
       v0[b][r] = l < nrows ? __ldcg(a.W + pty_tiled(row0 + l, j + r * F0::NR, a.rows, a.tl)) : make_float2(0.f, 0.f);
   }
   float2 v[FL::B][FL::R];
-  rfft<N, 0, true>(v0, v, smem, a.tw, cb);
+  rfft<N, 0, true, LD>(v0, v, smem, a.tw, cb);
   cp_wait<0>();
   __syncthreads();
   const float pmax = a.scal[0], omax = a.scal[1];

@@ -74,20 +74,37 @@ __device__ __forceinline__ bool bfly_of(int b, int cb, int& l, int& j) {
   return true;
 }
 
-// shared-memory word of element j + r*NR of line l (linear in r when NR % 16 == 0)
-template <int N, int NR>
-__device__ __forceinline__ int sidx_in(int l, int j, int r) {
+// Line stride of the row pass in float2.  A half-warp's 16 lanes take chunks of
+// 2^cb consecutive columns (cb the default chunk bits) on min(L, 16 / 2^cb) lines,
+// 16 / lines columns in all, so lines 16 / lines mod 16 apart put them on 16
+// different bank pairs; from cb = 4 on a half-warp stays on one line and the
+// column pass's stride (16 / L mod 16 for its line-fastest map) serves both.
+// Only 48 to 192 and 384 get a stride of their own (192^2 x96: 60.9 -> 46.8 us
+// per iteration, 384^2 x32: 60.8 -> 56.0).
+template <int N>
+__host__ __device__ constexpr int row_line_stride() {
   using G = Geom<N>;
-  if constexpr (NR % 16 == 0) return G::idx(l, j) + r * (NR + NR / 16);
-  else return G::idx(l, j + r * NR);
+  constexpr int cb = row_cb_pick(G::LOG2L, rfft_cb_max<N>());
+  if (cb >= 4) return G::LD;
+  const int lines = G::L < (16 >> cb) ? G::L : 16 >> cb;
+  return G::BASE + (((16 / lines - G::BASE) % 16) + 16) % 16;
+}
+
+// shared-memory word of element i of line l, lines LD words apart
+template <int LD>
+__device__ __forceinline__ int sidx(int l, int i) { return l * LD + i + (i >> 4); }
+// shared-memory word of element j + r*NR of line l (linear in r when NR % 16 == 0)
+template <int LD, int NR>
+__device__ __forceinline__ int sidx_in(int l, int j, int r) {
+  if constexpr (NR % 16 == 0) return sidx<LD>(l, j) + r * (NR + NR / 16);
+  else return sidx<LD>(l, j + r * NR);
 }
 // shared-memory word of element base + r*NS of line l
-template <int N, int R, int NS>
+template <int LD, int R, int NS>
 __device__ __forceinline__ int sidx_out(int l, int base, int r) {
-  using G = Geom<N>;
-  if constexpr (NS % 16 == 0) return G::idx(l, base) + r * (NS + NS / 16);
-  else if constexpr (NS == 1 && R == 16) return G::idx(l, base) + r;   // base = 16 j
-  else return G::idx(l, base + r * NS);
+  if constexpr (NS % 16 == 0) return sidx<LD>(l, base) + r * (NS + NS / 16);
+  else if constexpr (NS == 1 && R == 16) return sidx<LD>(l, base) + r;   // base = 16 j
+  else return sidx<LD>(l, base + r * NS);
 }
 
 // twiddles and the radix-R DFT of one butterfly of pass P
@@ -106,7 +123,7 @@ __device__ __forceinline__ void rpass_compute(float2 (&v)[RPass<N, PLAN, P>::R],
   dftR<S::R, INV>(v);
 }
 
-template <int N, int PLAN, int P>
+template <int N, int PLAN, int P, int LD>
 __device__ __forceinline__ void rpass_store(float2* buf, float2 (&v)[RPass<N, PLAN, P>::B][RPass<N, PLAN, P>::R],
                                             int cb) {
   using S = RPass<N, PLAN, P>;
@@ -117,11 +134,11 @@ __device__ __forceinline__ void rpass_store(float2* buf, float2 (&v)[RPass<N, PL
     const int k = j % S::NS;
     const int base = (j - k) * S::R + k;
 #pragma unroll
-    for (int r = 0; r < S::R; ++r) buf[sidx_out<N, S::R, S::NS>(l, base, r)] = v[b][r];
+    for (int r = 0; r < S::R; ++r) buf[sidx_out<LD, S::R, S::NS>(l, base, r)] = v[b][r];
   }
 }
 
-template <int N, int PLAN, int P>
+template <int N, int PLAN, int P, int LD>
 __device__ __forceinline__ void rpass_load(const float2* buf, float2 (&v)[RPass<N, PLAN, P>::B][RPass<N, PLAN, P>::R],
                                            int cb) {
   using S = RPass<N, PLAN, P>;
@@ -130,7 +147,7 @@ __device__ __forceinline__ void rpass_load(const float2* buf, float2 (&v)[RPass<
     int l, j;
     if (!bfly_of<N, S::R>(b, cb, l, j)) continue;
 #pragma unroll
-    for (int r = 0; r < S::R; ++r) v[b][r] = buf[sidx_in<N, S::NR>(l, j, r)];
+    for (int r = 0; r < S::R; ++r) v[b][r] = buf[sidx_in<LD, S::NR>(l, j, r)];
   }
 }
 
@@ -147,17 +164,17 @@ __device__ __forceinline__ void rpass_compute_all(float2 (&v)[RPass<N, PLAN, P>:
 }
 
 // middle passes P .. M-2 through shared memory (each ends with a barrier)
-template <int N, int PLAN, int P, bool INV>
+template <int N, int PLAN, int P, bool INV, int LD>
 __device__ __forceinline__ void rfft_middle(float2* buf, const float2* tw, int cb) {
   if constexpr (P < plan_len(N) - 1) {
     using S = RPass<N, PLAN, P>;
     float2 v[S::B][S::R];
-    rpass_load<N, PLAN, P>(buf, v, cb);
+    rpass_load<N, PLAN, P, LD>(buf, v, cb);
     __syncthreads();
     rpass_compute_all<N, PLAN, P, INV>(v, cb, tw);
-    rpass_store<N, PLAN, P>(buf, v, cb);
+    rpass_store<N, PLAN, P, LD>(buf, v, cb);
     __syncthreads();
-    rfft_middle<N, PLAN, P + 1, INV>(buf, tw, cb);
+    rfft_middle<N, PLAN, P + 1, INV, LD>(buf, tw, cb);
   }
 }
 
@@ -174,11 +191,12 @@ struct NoHook {
 // (element j + r*N/R0 of line l for butterfly (l, j)), `out` receives the
 // last pass's outputs (element j + r*NS_last).  The shared lines must be free
 // on entry (callers synchronise); on return other threads may still be
-// reading them, so callers synchronise before the next write.  `hook` runs
+// reading them, so callers synchronise before the next write.  LD: the line
+// stride of `buf` in float2.  `hook` runs
 // after every thread's last read of the shared lines has been issued and before
 // the last pass's arithmetic (a caller that synchronises there may refill the
 // lines while the last pass computes).
-template <int N, int PLAN, bool INV, class H = NoHook>
+template <int N, int PLAN, bool INV, int LD = Geom<N>::LD, class H = NoHook>
 __device__ __forceinline__ void rfft(float2 (&in)[RFirst<N, PLAN>::B][RFirst<N, PLAN>::R],
                                      float2 (&out)[RLast<N, PLAN>::B][RLast<N, PLAN>::R], float2* buf,
                                      const float2* tw, int cb, H&& hook = H{}) {
@@ -191,10 +209,10 @@ __device__ __forceinline__ void rfft(float2 (&in)[RFirst<N, PLAN>::B][RFirst<N, 
       for (int r = 0; r < RFirst<N, PLAN>::R; ++r) out[b][r] = in[b][r];
     hook();
   } else {
-    rpass_store<N, PLAN, 0>(buf, in, cb);
+    rpass_store<N, PLAN, 0, LD>(buf, in, cb);
     __syncthreads();
-    rfft_middle<N, PLAN, 1, INV>(buf, tw, cb);
-    rpass_load<N, PLAN, M - 1>(buf, out, cb);
+    rfft_middle<N, PLAN, 1, INV, LD>(buf, tw, cb);
+    rpass_load<N, PLAN, M - 1, LD>(buf, out, cb);
     hook();
     rpass_compute_all<N, PLAN, M - 1, INV>(out, cb, tw);
   }
@@ -226,8 +244,9 @@ template <int N>
 struct RGeom {
   using G = Geom<N>;
   static constexpr bool RHO_IN_BUF = CDX_RHO_IN_BUF && G::T == 256 && plan_len(N) > 1;
-  static constexpr int SMEM_ROW_ITER =
-      G::SMEM_LINES + (RHO_IN_BUF ? 0 : G::L * G::LD * (int)sizeof(float2)) + G::L * ((N + 31) >> 5) * 4;
+  static constexpr int ROW_LD = row_line_stride<N>();
+  static constexpr int SMEM_ROW_LINES = G::L * ROW_LD * (int)sizeof(float2);
+  static constexpr int SMEM_ROW_ITER = SMEM_ROW_LINES * (RHO_IN_BUF ? 1 : 2) + G::L * ((N + 31) >> 5) * 4;
   static constexpr int MINB_COL = (CDX_RK_MINB_COL > 0 && G::T == 256) ? CDX_RK_MINB_COL : G::MINB;
   static constexpr int MINB_ROW =
       (CDX_RK_MINB_ROW > 0 && G::T == 256) ? CDX_RK_MINB_ROW : (RHO_IN_BUF ? (N >= 1024 ? 3 : 4) : G::MINB);
@@ -427,7 +446,7 @@ __host__ __device__ constexpr bool row_sq_ok() { return Geom<N>::LOG2L <= rfft_c
 template <int N, int MODE, int ALGO, bool SQ = false>
 __device__ __forceinline__ void row_pass_body(const RowArgs& a) {
   using G = Geom<N>;
-  constexpr int L = G::L, T = G::T;
+  constexpr int L = G::L, T = G::T, LD = RGeom<N>::ROW_LD;
   using F0 = RFirst<N, 0>;
   using FL = RLast<N, 0>;
   using IL = RLast<N, 1>;
@@ -451,7 +470,7 @@ __device__ __forceinline__ void row_pass_body(const RowArgs& a) {
 
   // rho rows and support words of the CTA (ROW_ITER), landing during the inverse FFT
   // (RHO_IN_BUF: the rho rows land in the line buffer during its last pass)
-  constexpr int RS = G::LD;                 // rho line stride in shared memory
+  constexpr int RS = LD;                    // rho line stride in shared memory
   constexpr int WPR = (N + 31) >> 5;
   // Support words in shared memory: with MT the words a butterfly of the update
   // needs (columns j + r*NS, r < R: word (j >> 5) + r*NS/32) are staged next to
@@ -467,11 +486,12 @@ __device__ __forceinline__ void row_pass_body(const RowArgs& a) {
     }
   };
   constexpr bool rho_in_buf = RGeom<N>::RHO_IN_BUF;
-  float2* rho_s = rho_in_buf ? smem : smem + L * G::LD;
-  uint32_t* mask_s = reinterpret_cast<uint32_t*>(smem + L * G::LD + (rho_in_buf ? 0 : L * RS));
+  float2* rho_s = rho_in_buf ? smem : smem + L * LD;
+  uint32_t* mask_s = reinterpret_cast<uint32_t*>(smem + L * LD + (rho_in_buf ? 0 : L * RS));
   float2* rho = a.rho + (long long)blockIdx.y * a.rho_stride + (long long)row0 * N;
-  // with an even line stride each rho row is one bulk copy (16-byte aligned)
-  constexpr bool bulk_rho = bulk_staging<N>() && RS % 2 == 0;
+  // with an even line stride each rho row is one bulk copy (16-byte aligned); from 32 rows
+  // per CTA on, one thread issuing them is slower than 16-byte pieces by all (64^2: 14.4 -> 12.9 us)
+  constexpr bool bulk_rho = bulk_staging<N>() && RS % 2 == 0 && L <= 16;
   __shared__ uint64_t rho_bar;
   if constexpr (iter && bulk_rho) {
     if (threadIdx.x == 0) bulk_bar_init(&rho_bar);
@@ -541,15 +561,15 @@ __device__ __forceinline__ void row_pass_body(const RowArgs& a) {
       }
     }
     if constexpr (iter && rho_in_buf) {
-      rfft<N, 0, true>(v0, v, buf, tw, cb, [&]() {
+      rfft<N, 0, true, LD>(v0, v, buf, tw, cb, [&]() {
         __syncthreads();   // every thread's last read of the lines is done
         stage_rho();
         cp_commit();
       });
     } else if (iter || a.inv) {
-      rfft<N, 0, true>(v0, v, buf, tw, cb);
+      rfft<N, 0, true, LD>(v0, v, buf, tw, cb);
     } else {
-      rfft<N, 0, false>(v0, v, buf, tw, cb);
+      rfft<N, 0, false, LD>(v0, v, buf, tw, cb);
     }
   }
   float2* out = a.out + (long long)blockIdx.y * a.out_stride;
@@ -599,7 +619,7 @@ __device__ __forceinline__ void row_pass_body(const RowArgs& a) {
     }
     float2 o[IL::B][IL::R];
     if constexpr (rho_in_buf) __syncthreads();   // the rho rows are read before the lines are reused
-    rfft<N, 1, false>(v, o, buf, tw, cb);
+    rfft<N, 1, false, LD>(v, o, buf, tw, cb);
 #pragma unroll
     for (int b = 0; b < IL::B; ++b) {
       int l, j;

@@ -38,7 +38,7 @@ cudaError_t prepare_rk() {
   using G = Geom<N>;
   cudaError_t e;
   if ((e = cudaFuncSetAttribute(row_pass_rk<N, ROW_FFT, ALGO_ER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                G::SMEM_LINES)) != cudaSuccess)
+                                RGeom<N>::SMEM_ROW_LINES)) != cudaSuccess)
     return e;
   const void* iter_kernels[] = {
       (const void*)row_pass_rk<N, ROW_ITER, ALGO_HIO>, (const void*)row_pass_rk<N, ROW_ITER, ALGO_RAAR>,
@@ -98,7 +98,7 @@ cudaError_t launch_row(const RowArgs& a, int batch, cudaStream_t st) {
     else row_pass_kernel<N, ROW_FFT, 1><<<grid, G::T, G::SMEM_LINES, st>>>(a);
   } else {
     constexpr int SM = RGeom<N>::SMEM_ROW_ITER;
-    if (a.mode != ROW_ITER) return launch_pdl(row_pass_rk<N, ROW_FFT, ALGO_ER>, grid, G::T, G::SMEM_LINES, st, a, pdl_of<N>(a.pdl_mode));
+    if (a.mode != ROW_ITER) return launch_pdl(row_pass_rk<N, ROW_FFT, ALGO_ER>, grid, G::T, RGeom<N>::SMEM_ROW_LINES, st, a, pdl_of<N>(a.pdl_mode));
     if constexpr (row_sq_ok<N>()) if (row_sq_layout<N>(a)) switch (a.algo) {   // the compile-time layout of square patterns
       case ALGO_HIO: return launch_pdl(row_pass_rk<N, ROW_ITER, ALGO_HIO, true>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
       case ALGO_RAAR: return launch_pdl(row_pass_rk<N, ROW_ITER, ALGO_RAAR, true>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
