@@ -42,7 +42,7 @@ struct GemmArgs {
   const __nv_bfloat16* w;    // forward: W [Cout][K]; dgrad: Wt [Cin][K']
   float* out0;               // forward: Y; dgrad: dX part 0; wgrad: partials [split][Cout][K]
   float* out1;               // dgrad: dX part 1 (channels >= C0)
-  int accumulate;            // forward/dgrad: add into the output
+  int acc0, acc1;            // forward/dgrad: add into out0 / out1
   int m_per_split;           // wgrad: output pixels per split
 };
 
@@ -206,11 +206,12 @@ __global__ void __launch_bounds__(128) k_conv_gemm(GemmArgs a) {
           const int n = n0 + wn * WN + j * 8 + 2 * q + e;
           if (n >= NC) continue;
           const float v = acc[i][j][h * 2 + e];
+          const bool second = DGRAD && n >= s.C0;
           float* p;
           if (!DGRAD) p = a.out0 + (long long)m * s.Cout + n;
-          else if (n < s.C0) p = a.out0 + (long long)m * s.C0 + n;
+          else if (!second) p = a.out0 + (long long)m * s.C0 + n;
           else p = a.out1 + (long long)m * c1 + (n - s.C0);
-          *p = a.accumulate ? *p + v : v;
+          *p = (second ? a.acc1 : a.acc0) ? *p + v : v;
         }
     }
 }
@@ -353,7 +354,7 @@ struct ConvFwdOp {
   __device__ const void* dummy() const { return a.w; }
   __device__ void store(int m, int n0, const float* v, int cnt) const {
     float* p = a.out0 + (long long)m * a.s.Cout + n0;
-    for (int j = 0; j < cnt; ++j) p[j] = a.accumulate ? p[j] + v[j] : v[j];
+    for (int j = 0; j < cnt; ++j) p[j] = a.acc0 ? p[j] + v[j] : v[j];
   }
 };
 
@@ -395,7 +396,7 @@ struct ConvDgradOp {
     for (int j = 0; j < cnt; ++j) {
       const int n = n0 + j;
       float* p = n < s.C0 ? a.out0 + (long long)m * s.C0 + n : a.out1 + (long long)m * c1 + (n - s.C0);
-      *p = a.accumulate ? *p + v[j] : v[j];
+      *p = (n < s.C0 ? a.acc0 : a.acc1) ? *p + v[j] : v[j];
     }
   }
 };

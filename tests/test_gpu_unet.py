@@ -65,6 +65,32 @@ def test_gradients_match_fp64_oracle(cdx, torch_cuda, n, levels, base):
         assert rel(g[sl], g_ref[sl]) < 0.1, (d["kind"], d["wshape"], rel(g[sl], g_ref[sl]))
 
 
+@pytest.mark.parametrize("n,levels,base,groups,batch", [
+    (16, 2, 8, 8, 1),     # one channel per group, splits of a handful of pixels
+    (48, 2, 24, 3, 3),    # three octets of channels: idle threads, groups that stay single per CTA
+    (32, 2, 16, 2, 5),    # groups of 8 and 16 channels
+    (64, 3, 64, 8, 2),    # groups of 32 channels and more than a CTA's 32
+])
+def test_group_norm_geometries_match_oracle(cdx, torch_cuda, n, levels, base, groups, batch):
+    """Channel and group splits of the GroupNorm, input and loss kernels, with the bounds of
+    test_gradients_match_fp64_oracle."""
+    torch = torch_cuda
+    from cdixx_gb300 import unet
+    I, amp, ph, sup = small_case(n, batch, seed=9)
+    p = U.init_params(n, levels, base, seed=11)
+    loss_ref, g_ref, out_ref = U.forward_backward(p, I, amp, ph, sup, n, levels, base, groups=groups, round_bf16=True)
+    with unet.UNet(n=n, levels=levels, base=base, batch=batch, groups=groups) as net:
+        net.set_params(p)
+        dev = [torch.from_numpy(x).cuda() for x in (I, amp, ph, sup)]
+        out = net.forward(dev[0]).cpu().numpy().transpose(0, 2, 3, 1)
+        loss = net.loss_backward(*dev)
+        g = net.grads().astype(np.float64)
+    rel = lambda a, b: np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-30)
+    assert rel(out, out_ref) < 5e-3
+    assert abs(loss - loss_ref) <= 2e-3 * abs(loss_ref)
+    assert rel(g, g_ref) < 3e-2
+
+
 def test_forward_model_matches_restatement(cdx, torch_cuda):
     from cdixx_gb300 import unet
     n, count, seed, first = 64, 3, 11, 5
