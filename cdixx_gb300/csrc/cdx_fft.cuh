@@ -269,16 +269,12 @@ __host__ __device__ constexpr int pow2_floor(int x) {
   return p;
 }
 
-// Launch geometry per length: T threads, L lines per CTA (a power of two >= 2,
-// so a tile of L columns has a power-of-two width and a row CTA moves at least
-// 32-byte pieces of it), about 16 complex values per thread and pass (32 at
-// N = 4096).  Small CTAs keep three or more resident per SM.
-template <int N>
-struct Geom {
-  static constexpr int T = N >= 3072 ? 512 : 256;
-  static constexpr int MINB = T == 512 ? 1 : 3;   // resident CTAs per SM the register budget targets
-  static constexpr int ELEMS = 16 * T;
-  static constexpr int L = pow2_floor((ELEMS / N) < 2 ? 2 : (ELEMS / N));
+// Launch geometry of a pass: T threads hold L lines of length N (a power of two
+// >= 2), about 16 complex values per thread and pass.
+template <int N_, int T_, int L_>
+struct GeomT {
+  static constexpr int N = N_, T = T_, L = L_;
+  static constexpr int MINB = T >= 512 ? 1 : 3;   // resident CTAs per SM the register budget targets
   static constexpr int LOG2L = L == 1 ? 0 : (L == 2 ? 1 : (L == 4 ? 2 : (L == 8 ? 3 : (L == 16 ? 4 : (L == 32 ? 5 :
                                (L == 64 ? 6 : (L == 128 ? 7 : 8)))))));
   // line stride in float2: >= N + N/16, and for L < 16 congruent to 16/L mod 16
@@ -297,6 +293,13 @@ struct Geom {
   static constexpr int SMEM_MAX = SMEM_ROW_ITER > SMEM_COL_CCD ? SMEM_ROW_ITER : SMEM_COL_CCD;
   __device__ __forceinline__ static int idx(int l, int i) { return l * LD + i + (i >> 4); }
 };
+// The geometry of length N: tiles of L columns have a power-of-two width and a
+// row CTA moves at least 32-byte pieces of them; small CTAs keep three or more
+// resident per SM (512 threads at 3072 and 4096).
+constexpr int geom_t(int n) { return n >= 3072 ? 512 : 256; }
+constexpr int geom_l(int n) { return pow2_floor((16 * geom_t(n) / n) < 2 ? 2 : (16 * geom_t(n) / n)); }
+template <int N>
+struct Geom : GeomT<N, geom_t(N), geom_l(N)> {};
 
 // One Stockham pass over the L lines of Geom<N>.
 template <int N, int P, bool INV>

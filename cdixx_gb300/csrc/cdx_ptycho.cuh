@@ -114,8 +114,8 @@ template <int N>
 struct PtyRow {
   static constexpr int SN = N + 8;
   static constexpr int STAGE = 2 * Geom<N>::L * SN * (int)sizeof(float2);
-  static constexpr int LD = RGeom<N>::ROW_LD;
-  static constexpr int SMEM = RGeom<N>::SMEM_ROW_LINES + STAGE;
+  static constexpr int LD = RGeom<Geom<N>>::ROW_LD;
+  static constexpr int SMEM = RGeom<Geom<N>>::SMEM_ROW_LINES + STAGE;
 };
 
 template <int N>
@@ -142,8 +142,8 @@ template <int N, bool FRES>
 __global__ void __launch_bounds__(Geom<N>::T, Geom<N>::MINB) pty_fwd_rk(PtyArgs a) {
   using G = Geom<N>;
   constexpr int L = G::L;
-  using F0 = RFirst<N, 0>;
-  using FL = RLast<N, 0>;
+  using F0 = RFirst<G, 0>;
+  using FL = RLast<G, 0>;
   constexpr int SN = PtyRow<N>::SN, LD = PtyRow<N>::LD;
   extern __shared__ float2 smem[];
   pdl_wait_and_release();
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(Geom<N>::T, Geom<N>::MINB) pty_fwd_rk(PtyArgs 
 #pragma unroll
   for (int b = 0; b < F0::B; ++b) {
     int l, j;
-    if (!bfly_of<N, F0::R>(b, cb, l, j)) continue;
+    if (!bfly_of<G, F0::R>(b, cb, l, j)) continue;
 #pragma unroll
     for (int r = 0; r < F0::R; ++r) {
       const int t = l * SN + j + r * F0::NR;   // multiply(esw, probe, window): zero outside the object
@@ -169,11 +169,11 @@ __global__ void __launch_bounds__(Geom<N>::T, Geom<N>::MINB) pty_fwd_rk(PtyArgs 
     }
   }
   float2 v[FL::B][FL::R];
-  rfft<N, 0, false, LD>(v0, v, smem, a.tw, cb);
+  rfft<G, 0, false, LD>(v0, v, smem, a.tw, cb);
 #pragma unroll
   for (int b = 0; b < FL::B; ++b) {
     int l, j;
-    if (!bfly_of<N, FL::R>(b, cb, l, j) || l >= nrows) continue;
+    if (!bfly_of<G, FL::R>(b, cb, l, j) || l >= nrows) continue;
 #pragma unroll
     for (int r = 0; r < FL::R; ++r) __stcg(a.W + pty_tiled(row0 + l, j + r * FL::NS, a.rows, a.tl), v[b][r]);
   }
@@ -181,12 +181,12 @@ __global__ void __launch_bounds__(Geom<N>::T, Geom<N>::MINB) pty_fwd_rk(PtyArgs 
 
 // ------------------------------------------------------------ column pass
 template <int N>
-__global__ void __launch_bounds__(Geom<N>::T, RGeom<N>::MINB_COL) pty_col_rk(PtyArgs a) {
+__global__ void __launch_bounds__(Geom<N>::T, RGeom<Geom<N>>::MINB_COL) pty_col_rk(PtyArgs a) {
   using G = Geom<N>;
   constexpr int L = G::L, T = G::T;
-  using F0 = RFirst<N, 0>;
-  using FL = RLast<N, 0>;
-  using IL = RLast<N, 1>;
+  using F0 = RFirst<G, 0>;
+  using FL = RLast<G, 0>;
+  using IL = RLast<G, 1>;
   extern __shared__ float2 smem[];
   pdl_wait_and_release();
   const int c0 = blockIdx.x * L;
@@ -220,19 +220,19 @@ __global__ void __launch_bounds__(Geom<N>::T, RGeom<N>::MINB_COL) pty_col_rk(Pty
 #pragma unroll
   for (int b = 0; b < F0::B; ++b) {
     int l, j;
-    if (!bfly_of<N, F0::R>(b, 0, l, j)) continue;
+    if (!bfly_of<G, F0::R>(b, 0, l, j)) continue;
 #pragma unroll
     for (int r = 0; r < F0::R; ++r) v0[b][r] = __ldcg(a.W + tile + (long long)(j + r * F0::NR) * L + l);
   }
   float2 v[FL::B][FL::R];
-  rfft<N, 0, false>(v0, v, smem, a.tw, 0);
+  rfft<G, 0, false>(v0, v, smem, a.tw, 0);
   if constexpr (bulk_staging<N>()) bulk_wait(&stage_bar, a.err);
   else cp_wait<0>();
   __syncthreads();
 #pragma unroll
   for (int b = 0; b < FL::B; ++b) {
     int l, j;
-    if (!bfly_of<N, FL::R>(b, 0, l, j)) continue;
+    if (!bfly_of<G, FL::R>(b, 0, l, j)) continue;
 #pragma unroll
     for (int r = 0; r < FL::R; ++r) {
       const int t = (j + r * FL::NS) * L + l;
@@ -244,11 +244,11 @@ __global__ void __launch_bounds__(Geom<N>::T, RGeom<N>::MINB_COL) pty_col_rk(Pty
     }
   }
   float2 o[IL::B][IL::R];
-  rfft<N, 1, true>(v, o, smem, a.tw, 0);
+  rfft<G, 1, true>(v, o, smem, a.tw, 0);
 #pragma unroll
   for (int b = 0; b < IL::B; ++b) {
     int l, j;
-    if (!bfly_of<N, IL::R>(b, 0, l, j)) continue;
+    if (!bfly_of<G, IL::R>(b, 0, l, j)) continue;
 #pragma unroll
     for (int r = 0; r < IL::R; ++r) __stcg(a.W + tile + (long long)(j + r * IL::NS) * L + l, o[b][r]);
   }
@@ -259,8 +259,8 @@ template <int N, bool FRES>
 __global__ void __launch_bounds__(Geom<N>::T, Geom<N>::MINB) pty_upd_rk(PtyArgs a) {
   using G = Geom<N>;
   constexpr int L = G::L;
-  using F0 = RFirst<N, 0>;
-  using FL = RLast<N, 0>;
+  using F0 = RFirst<G, 0>;
+  using FL = RLast<G, 0>;
   constexpr int SN = PtyRow<N>::SN, LD = PtyRow<N>::LD;
   extern __shared__ float2 smem[];
   pdl_wait_and_release();
@@ -277,20 +277,20 @@ __global__ void __launch_bounds__(Geom<N>::T, Geom<N>::MINB) pty_upd_rk(PtyArgs 
 #pragma unroll
   for (int b = 0; b < F0::B; ++b) {
     int l, j;
-    if (!bfly_of<N, F0::R>(b, cb, l, j)) continue;
+    if (!bfly_of<G, F0::R>(b, cb, l, j)) continue;
 #pragma unroll
     for (int r = 0; r < F0::R; ++r)
       v0[b][r] = l < nrows ? __ldcg(a.W + pty_tiled(row0 + l, j + r * F0::NR, a.rows, a.tl)) : make_float2(0.f, 0.f);
   }
   float2 v[FL::B][FL::R];
-  rfft<N, 0, true, LD>(v0, v, smem, a.tw, cb);
+  rfft<G, 0, true, LD>(v0, v, smem, a.tw, cb);
   cp_wait<0>();
   __syncthreads();
   const float pmax = a.scal[0], omax = a.scal[1];
 #pragma unroll
   for (int b = 0; b < FL::B; ++b) {
     int l, j;
-    if (!bfly_of<N, FL::R>(b, cb, l, j) || l >= nrows) continue;
+    if (!bfly_of<G, FL::R>(b, cb, l, j) || l >= nrows) continue;
 #pragma unroll
     for (int r = 0; r < FL::R; ++r) {
       const int c = j + r * FL::NS, row = row0 + l;

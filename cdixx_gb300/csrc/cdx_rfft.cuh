@@ -27,9 +27,9 @@
 
 namespace cdx {
 
-template <int N, int PLAN, int P>
+template <class G, int PLAN, int P>
 struct RPass {
-  using G = Geom<N>;
+  static constexpr int N = G::N;
   static constexpr int R = plan_radix_x(N, PLAN, P);
   static constexpr int NS = plan_ns_x(N, PLAN, P);
   static constexpr int NR = N / R;
@@ -63,10 +63,9 @@ __host__ __device__ constexpr int rfft_cb_max() {
 }
 
 // (l, j) of butterfly b of this thread in a radix-R pass; false past the end
-template <int N, int R>
+template <class G, int R>
 __device__ __forceinline__ bool bfly_of(int b, int cb, int& l, int& j) {
-  using G = Geom<N>;
-  constexpr int NB = G::L * (N / R);
+  constexpr int NB = G::L * (G::N / R);
   const int g = threadIdx.x + b * G::T;
   if ((NB % G::T) != 0 && g >= NB) return false;
   l = (g >> cb) & (G::L - 1);
@@ -81,10 +80,9 @@ __device__ __forceinline__ bool bfly_of(int b, int cb, int& l, int& j) {
 // column pass's stride (16 / L mod 16 for its line-fastest map) serves both.
 // Only 48 to 192 and 384 get a stride of their own (192^2 x96: 60.9 -> 46.8 us
 // per iteration, 384^2 x32: 60.8 -> 56.0).
-template <int N>
+template <class G>
 __host__ __device__ constexpr int row_line_stride() {
-  using G = Geom<N>;
-  constexpr int cb = row_cb_pick(G::LOG2L, rfft_cb_max<N>());
+  constexpr int cb = row_cb_pick(G::LOG2L, rfft_cb_max<G::N>());
   if (cb >= 4) return G::LD;
   const int lines = G::L < (16 >> cb) ? G::L : 16 >> cb;
   return G::BASE + (((16 / lines - G::BASE) % 16) + 16) % 16;
@@ -108,9 +106,9 @@ __device__ __forceinline__ int sidx_out(int l, int base, int r) {
 }
 
 // twiddles and the radix-R DFT of one butterfly of pass P
-template <int N, int PLAN, int P, bool INV>
-__device__ __forceinline__ void rpass_compute(float2 (&v)[RPass<N, PLAN, P>::R], int j, const float2* tw) {
-  using S = RPass<N, PLAN, P>;
+template <class G, int PLAN, int P, bool INV>
+__device__ __forceinline__ void rpass_compute(float2 (&v)[RPass<G, PLAN, P>::R], int j, const float2* tw) {
+  using S = RPass<G, PLAN, P>;
   if constexpr (S::NS > 1) {
     const int k = j % S::NS;
 #pragma unroll
@@ -123,14 +121,14 @@ __device__ __forceinline__ void rpass_compute(float2 (&v)[RPass<N, PLAN, P>::R],
   dftR<S::R, INV>(v);
 }
 
-template <int N, int PLAN, int P, int LD>
-__device__ __forceinline__ void rpass_store(float2* buf, float2 (&v)[RPass<N, PLAN, P>::B][RPass<N, PLAN, P>::R],
+template <class G, int PLAN, int P, int LD>
+__device__ __forceinline__ void rpass_store(float2* buf, float2 (&v)[RPass<G, PLAN, P>::B][RPass<G, PLAN, P>::R],
                                             int cb) {
-  using S = RPass<N, PLAN, P>;
+  using S = RPass<G, PLAN, P>;
 #pragma unroll
   for (int b = 0; b < S::B; ++b) {
     int l, j;
-    if (!bfly_of<N, S::R>(b, cb, l, j)) continue;
+    if (!bfly_of<G, S::R>(b, cb, l, j)) continue;
     const int k = j % S::NS;
     const int base = (j - k) * S::R + k;
 #pragma unroll
@@ -138,50 +136,50 @@ __device__ __forceinline__ void rpass_store(float2* buf, float2 (&v)[RPass<N, PL
   }
 }
 
-template <int N, int PLAN, int P, int LD>
-__device__ __forceinline__ void rpass_load(const float2* buf, float2 (&v)[RPass<N, PLAN, P>::B][RPass<N, PLAN, P>::R],
+template <class G, int PLAN, int P, int LD>
+__device__ __forceinline__ void rpass_load(const float2* buf, float2 (&v)[RPass<G, PLAN, P>::B][RPass<G, PLAN, P>::R],
                                            int cb) {
-  using S = RPass<N, PLAN, P>;
+  using S = RPass<G, PLAN, P>;
 #pragma unroll
   for (int b = 0; b < S::B; ++b) {
     int l, j;
-    if (!bfly_of<N, S::R>(b, cb, l, j)) continue;
+    if (!bfly_of<G, S::R>(b, cb, l, j)) continue;
 #pragma unroll
     for (int r = 0; r < S::R; ++r) v[b][r] = buf[sidx_in<LD, S::NR>(l, j, r)];
   }
 }
 
-template <int N, int PLAN, int P, bool INV>
-__device__ __forceinline__ void rpass_compute_all(float2 (&v)[RPass<N, PLAN, P>::B][RPass<N, PLAN, P>::R], int cb,
+template <class G, int PLAN, int P, bool INV>
+__device__ __forceinline__ void rpass_compute_all(float2 (&v)[RPass<G, PLAN, P>::B][RPass<G, PLAN, P>::R], int cb,
                                                   const float2* tw) {
-  using S = RPass<N, PLAN, P>;
+  using S = RPass<G, PLAN, P>;
 #pragma unroll
   for (int b = 0; b < S::B; ++b) {
     int l, j;
-    if (!bfly_of<N, S::R>(b, cb, l, j)) continue;
-    rpass_compute<N, PLAN, P, INV>(v[b], j, tw);
+    if (!bfly_of<G, S::R>(b, cb, l, j)) continue;
+    rpass_compute<G, PLAN, P, INV>(v[b], j, tw);
   }
 }
 
 // middle passes P .. M-2 through shared memory (each ends with a barrier)
-template <int N, int PLAN, int P, bool INV, int LD>
+template <class G, int PLAN, int P, bool INV, int LD>
 __device__ __forceinline__ void rfft_middle(float2* buf, const float2* tw, int cb) {
-  if constexpr (P < plan_len(N) - 1) {
-    using S = RPass<N, PLAN, P>;
+  if constexpr (P < plan_len(G::N) - 1) {
+    using S = RPass<G, PLAN, P>;
     float2 v[S::B][S::R];
-    rpass_load<N, PLAN, P, LD>(buf, v, cb);
+    rpass_load<G, PLAN, P, LD>(buf, v, cb);
     __syncthreads();
-    rpass_compute_all<N, PLAN, P, INV>(v, cb, tw);
-    rpass_store<N, PLAN, P, LD>(buf, v, cb);
+    rpass_compute_all<G, PLAN, P, INV>(v, cb, tw);
+    rpass_store<G, PLAN, P, LD>(buf, v, cb);
     __syncthreads();
-    rfft_middle<N, PLAN, P + 1, INV, LD>(buf, tw, cb);
+    rfft_middle<G, PLAN, P + 1, INV, LD>(buf, tw, cb);
   }
 }
 
-template <int N, int PLAN>
-using RFirst = RPass<N, PLAN, 0>;
-template <int N, int PLAN>
-using RLast = RPass<N, PLAN, plan_len(N) - 1>;
+template <class G, int PLAN>
+using RFirst = RPass<G, PLAN, 0>;
+template <class G, int PLAN>
+using RLast = RPass<G, PLAN, plan_len(G::N) - 1>;
 
 struct NoHook {
   __device__ __forceinline__ void operator()() const {}
@@ -196,25 +194,25 @@ struct NoHook {
 // after every thread's last read of the shared lines has been issued and before
 // the last pass's arithmetic (a caller that synchronises there may refill the
 // lines while the last pass computes).
-template <int N, int PLAN, bool INV, int LD = Geom<N>::LD, class H = NoHook>
-__device__ __forceinline__ void rfft(float2 (&in)[RFirst<N, PLAN>::B][RFirst<N, PLAN>::R],
-                                     float2 (&out)[RLast<N, PLAN>::B][RLast<N, PLAN>::R], float2* buf,
+template <class G, int PLAN, bool INV, int LD = G::LD, class H = NoHook>
+__device__ __forceinline__ void rfft(float2 (&in)[RFirst<G, PLAN>::B][RFirst<G, PLAN>::R],
+                                     float2 (&out)[RLast<G, PLAN>::B][RLast<G, PLAN>::R], float2* buf,
                                      const float2* tw, int cb, H&& hook = H{}) {
-  constexpr int M = plan_len(N);
-  rpass_compute_all<N, PLAN, 0, INV>(in, cb, tw);
+  constexpr int M = plan_len(G::N);
+  rpass_compute_all<G, PLAN, 0, INV>(in, cb, tw);
   if constexpr (M == 1) {
 #pragma unroll
-    for (int b = 0; b < RFirst<N, PLAN>::B; ++b)
+    for (int b = 0; b < RFirst<G, PLAN>::B; ++b)
 #pragma unroll
-      for (int r = 0; r < RFirst<N, PLAN>::R; ++r) out[b][r] = in[b][r];
+      for (int r = 0; r < RFirst<G, PLAN>::R; ++r) out[b][r] = in[b][r];
     hook();
   } else {
-    rpass_store<N, PLAN, 0, LD>(buf, in, cb);
+    rpass_store<G, PLAN, 0, LD>(buf, in, cb);
     __syncthreads();
-    rfft_middle<N, PLAN, 1, INV, LD>(buf, tw, cb);
-    rpass_load<N, PLAN, M - 1, LD>(buf, out, cb);
+    rfft_middle<G, PLAN, 1, INV, LD>(buf, tw, cb);
+    rpass_load<G, PLAN, M - 1, LD>(buf, out, cb);
     hook();
-    rpass_compute_all<N, PLAN, M - 1, INV>(out, cb, tw);
+    rpass_compute_all<G, PLAN, M - 1, INV>(out, cb, tw);
   }
 }
 
@@ -240,17 +238,28 @@ __device__ __forceinline__ void rfft(float2 (&in)[RFirst<N, PLAN>::B][RFirst<N, 
 #ifndef CDX_RHO_IN_BUF
 #define CDX_RHO_IN_BUF 1
 #endif
-template <int N>
+template <class G>
 struct RGeom {
-  using G = Geom<N>;
+  static constexpr int N = G::N;
   static constexpr bool RHO_IN_BUF = CDX_RHO_IN_BUF && G::T == 256 && plan_len(N) > 1;
-  static constexpr int ROW_LD = row_line_stride<N>();
+  static constexpr int ROW_LD = row_line_stride<G>();
   static constexpr int SMEM_ROW_LINES = G::L * ROW_LD * (int)sizeof(float2);
   static constexpr int SMEM_ROW_ITER = SMEM_ROW_LINES * (RHO_IN_BUF ? 1 : 2) + G::L * ((N + 31) >> 5) * 4;
-  static constexpr int MINB_COL = (CDX_RK_MINB_COL > 0 && G::T == 256) ? CDX_RK_MINB_COL : G::MINB;
+  static constexpr int MINB_COL = (CDX_RK_MINB_COL > 0 && G::T == 256) ? CDX_RK_MINB_COL : (G::T == 512 ? 2 : 1);
   static constexpr int MINB_ROW =
       (CDX_RK_MINB_ROW > 0 && G::T == 256) ? CDX_RK_MINB_ROW : (RHO_IN_BUF ? (N >= 1024 ? 3 : 4) : G::MINB);
+  static constexpr int MINB_ROW_FFT = G::T == 512 ? 2 : MINB_ROW;
 };
+// Geometry of a column transform alone whose output is row-major: the default
+// tiles of 2 or 4 columns read and write 16- or 32-byte pieces of each row, so the
+// lengths from 1024 up take WIDE_L columns in a CTA of WIDE_L N / 16 threads where
+// there are enough of them for every SM (whole transform: 4096^2 197 -> 140 us,
+// 3072^2 123 -> 95, 2048^2 46.0 -> 37.0, 1024^2 x8 61.7 -> 57.4; 4 columns at 2048^2
+// 39.5; 8 at 768^2 x8 35.4 -> 38.3, so 768 keeps its own).  Two CTAs of 512 threads
+// per SM in the row transforms of 3072 and 4096 are part of it.
+constexpr int wide_l(int n) { return n >= 3072 ? 4 : (n >= 1024 ? 8 : geom_l(n)); }
+template <int N>
+struct WideGeom : GeomT<N, wide_l(N) == geom_l(N) ? geom_t(N) : wide_l(N) * N / 16, wide_l(N)> {};
 
 // ------------------------------------------------------------- real-space updates
 template <int ALGO>
@@ -261,14 +270,16 @@ __device__ __forceinline__ float2 update_t(bool inside, float2 x, float2 p, floa
 // ---------------------------------------------------------------- column pass
 // Lines are columns (length N = rows).  Column-tiled arrays have tile width L.
 // PROJ (COL_ITER): the modulus projection, PROJ_MODABS or PROJ_CCD.
-template <int N, int MODE, int PROJ>
-__global__ void __launch_bounds__(Geom<N>::T, RGeom<N>::MINB_COL) col_pass_rk(ColArgs a) {
-  using G = Geom<N>;
-  constexpr int L = G::L, T = G::T;
-  using F0 = RFirst<N, 0>;
-  using FL = RLast<N, 0>;   // == RFirst<N, 1> in shape
-  using IL = RLast<N, 1>;
-  static_assert(FL::R == RFirst<N, 1>::R && FL::B == RFirst<N, 1>::B, "plan 1 starts where plan 0 ends");
+// TL: log2 of the tile width of column-tiled data (COL_FFT on a wide geometry:
+// narrower than the CTA's L columns).
+template <class G, int MODE, int PROJ, int TL = G::LOG2L>
+__global__ void __launch_bounds__(G::T, RGeom<G>::MINB_COL) col_pass_rk(ColArgs a) {
+  constexpr int N = G::N, L = G::L, T = G::T;
+  static_assert(TL == G::LOG2L || MODE == COL_FFT, "the iteration's tiles are as wide as its CTAs");
+  using F0 = RFirst<G, 0>;
+  using FL = RLast<G, 0>;   // == RFirst<G, 1> in shape
+  using IL = RLast<G, 1>;
+  static_assert(FL::R == RFirst<G, 1>::R && FL::B == RFirst<G, 1>::B, "plan 1 starts where plan 0 ends");
   extern __shared__ float2 smem[];
   __shared__ double red[T / 32];
   pdl_wait_and_release();
@@ -321,7 +332,12 @@ __global__ void __launch_bounds__(Geom<N>::T, RGeom<N>::MINB_COL) col_pass_rk(Co
   const float2* in = a.in + (long long)blockIdx.y * a.in_stride;
   const bool in_t = a.in_tiled != 0;
   auto gload = [&](int l, int m) -> float2 {
-    if (in_t) return __ldcg(in + tile + (long long)m * L + l);
+    if constexpr (TL == G::LOG2L) {
+      if (in_t) return __ldcg(in + tile + (long long)m * L + l);
+    } else {
+      if (in_t && l < ncols)   // tile (c0 + l) >> TL of the CTA's columns
+        return __ldcg(in + tile + (long long)(l >> TL) * (N << TL) + (m << TL) + (l & ((1 << TL) - 1)));
+    }
     return l < ncols ? __ldcg(in + m * C + c0 + l) : make_float2(0.f, 0.f);
   };
   float2 v[FL::B][FL::R];
@@ -331,18 +347,18 @@ __global__ void __launch_bounds__(Geom<N>::T, RGeom<N>::MINB_COL) col_pass_rk(Co
 #pragma unroll
     for (int b = 0; b < F0::B; ++b) {
       int l, j;
-      if (!bfly_of<N, F0::R>(b, 0, l, j)) continue;
+      if (!bfly_of<G, F0::R>(b, 0, l, j)) continue;
 #pragma unroll
       for (int r = 0; r < F0::R; ++r) v0[b][r] = gload(l, j + r * F0::NR);
     }
-    if (!iter && a.inv) rfft<N, 0, true>(v0, v, buf, tw, 0);
-    else rfft<N, 0, false>(v0, v, buf, tw, 0);
+    if (!iter && a.inv) rfft<G, 0, true>(v0, v, buf, tw, 0);
+    else rfft<G, 0, false>(v0, v, buf, tw, 0);
   } else {
     // Psi given: load it where the forward transform would have left it
 #pragma unroll
     for (int b = 0; b < FL::B; ++b) {
       int l, j;
-      if (!bfly_of<N, FL::R>(b, 0, l, j)) continue;
+      if (!bfly_of<G, FL::R>(b, 0, l, j)) continue;
 #pragma unroll
       for (int r = 0; r < FL::R; ++r) v[b][r] = gload(l, j + r * FL::NS);
     }
@@ -354,13 +370,13 @@ __global__ void __launch_bounds__(Geom<N>::T, RGeom<N>::MINB_COL) col_pass_rk(Co
 #pragma unroll
     for (int b = 0; b < FL::B; ++b) {
       int l, j;
-      if (!bfly_of<N, FL::R>(b, 0, l, j)) continue;
+      if (!bfly_of<G, FL::R>(b, 0, l, j)) continue;
 #pragma unroll
       for (int r = 0; r < FL::R; ++r) {
         const int m = j + r * FL::NS;
         float2 y = v[b][r];
         if (s != 1.f) { y.x *= s; y.y *= s; }
-        if (out_t) __stcg(out + tile + (long long)m * L + l, y);
+        if (TL == G::LOG2L && out_t) __stcg(out + tile + (long long)m * L + l, y);
         else if (l < ncols) __stcg(out + m * C + c0 + l, y);
       }
     }
@@ -377,7 +393,7 @@ __global__ void __launch_bounds__(Geom<N>::T, RGeom<N>::MINB_COL) col_pass_rk(Co
 #pragma unroll
       for (int b = 0; b < FL::B; ++b) {
         int l, j;
-        if (!bfly_of<N, FL::R>(b, 0, l, j) || l >= ncols) continue;
+        if (!bfly_of<G, FL::R>(b, 0, l, j) || l >= ncols) continue;
 #pragma unroll
         for (int r = 0; r < FL::R; ++r) {
           const float2 z = v[b][r];
@@ -390,7 +406,7 @@ __global__ void __launch_bounds__(Geom<N>::T, RGeom<N>::MINB_COL) col_pass_rk(Co
 #pragma unroll
     for (int b = 0; b < FL::B; ++b) {
       int l, j;
-      if (!bfly_of<N, FL::R>(b, 0, l, j)) continue;
+      if (!bfly_of<G, FL::R>(b, 0, l, j)) continue;
 #pragma unroll
       for (int r = 0; r < FL::R; ++r) {
         const int t = (j + r * FL::NS) * L + l;
@@ -406,17 +422,17 @@ __global__ void __launch_bounds__(Geom<N>::T, RGeom<N>::MINB_COL) col_pass_rk(Co
 #pragma unroll
       for (int b = 0; b < FL::B; ++b) {
         int l, j;
-        if (!bfly_of<N, FL::R>(b, 0, l, j) || l >= ncols) continue;
+        if (!bfly_of<G, FL::R>(b, 0, l, j) || l >= ncols) continue;
 #pragma unroll
         for (int r = 0; r < FL::R; ++r) psi_out[(j + r * FL::NS) * C + c0 + l] = v[b][r];
       }
     }
     float2 o[IL::B][IL::R];
-    rfft<N, 1, true>(v, o, buf, tw, 0);
+    rfft<G, 1, true>(v, o, buf, tw, 0);
 #pragma unroll
     for (int b = 0; b < IL::B; ++b) {
       int l, j;
-      if (!bfly_of<N, IL::R>(b, 0, l, j)) continue;
+      if (!bfly_of<G, IL::R>(b, 0, l, j)) continue;
 #pragma unroll
       for (int r = 0; r < IL::R; ++r) {
         const int m = j + r * IL::NS;
@@ -440,24 +456,25 @@ __global__ void __launch_bounds__(Geom<N>::T, RGeom<N>::MINB_COL) col_pass_rk(Co
 // The compile-time layout needs every pass's element stride to be whole tiles:
 // 2^log2(L) divides N/R for each radix R (true from 256 up; at 16..192 the
 // column tiles are wider than that).
+template <class G>
+__host__ __device__ constexpr bool row_sq_ok_g() { return G::LOG2L <= rfft_cb_max<G::N>(); }
 template <int N>
-__host__ __device__ constexpr bool row_sq_ok() { return Geom<N>::LOG2L <= rfft_cb_max<N>(); }
+__host__ __device__ constexpr bool row_sq_ok() { return row_sq_ok_g<Geom<N>>(); }
 
-template <int N, int MODE, int ALGO, bool SQ = false>
+template <class G, int MODE, int ALGO, bool SQ = false>
 __device__ __forceinline__ void row_pass_body(const RowArgs& a) {
-  using G = Geom<N>;
-  constexpr int L = G::L, T = G::T, LD = RGeom<N>::ROW_LD;
-  using F0 = RFirst<N, 0>;
-  using FL = RLast<N, 0>;
-  using IL = RLast<N, 1>;
-  static_assert(FL::R == RFirst<N, 1>::R && FL::B == RFirst<N, 1>::B, "plan 1 starts where plan 0 ends");
+  constexpr int N = G::N, L = G::L, T = G::T, LD = RGeom<G>::ROW_LD;
+  using F0 = RFirst<G, 0>;
+  using FL = RLast<G, 0>;
+  using IL = RLast<G, 1>;
+  static_assert(FL::R == RFirst<G, 1>::R && FL::B == RFirst<G, 1>::B, "plan 1 starts where plan 0 ends");
   extern __shared__ float2 smem[];
   const float2* __restrict__ tw = a.tw;
   float2* buf = smem;
   const int row0 = blockIdx.x * L;
   const int nrows = min(L, a.rows - row0);
   constexpr bool iter = MODE == ROW_ITER;
-  constexpr bool CT = SQ && iter && row_sq_ok<N>();   // compile-time layout
+  constexpr bool CT = SQ && iter && row_sq_ok_g<G>();   // compile-time layout
   constexpr int TLC = G::LOG2L;
   constexpr int CBC = row_cb_pick(TLC, rfft_cb_max<N>());
   const int tl = CT ? TLC : a.tile_log2;
@@ -485,7 +502,7 @@ __device__ __forceinline__ void row_pass_body(const RowArgs& a) {
       return w;
     }
   };
-  constexpr bool rho_in_buf = RGeom<N>::RHO_IN_BUF;
+  constexpr bool rho_in_buf = RGeom<G>::RHO_IN_BUF;
   float2* rho_s = rho_in_buf ? smem : smem + L * LD;
   uint32_t* mask_s = reinterpret_cast<uint32_t*>(smem + L * LD + (rho_in_buf ? 0 : L * RS));
   float2* rho = a.rho + (long long)blockIdx.y * a.rho_stride + (long long)row0 * N;
@@ -546,7 +563,7 @@ __device__ __forceinline__ void row_pass_body(const RowArgs& a) {
 #pragma unroll
     for (int b = 0; b < F0::B; ++b) {
       int l, j;
-      if (!bfly_of<N, F0::R>(b, cb, l, j)) continue;
+      if (!bfly_of<G, F0::R>(b, cb, l, j)) continue;
       if constexpr (CT) {
         // element j + r*NR: tile (j >> TLC) + r*(NR >> TLC), lane j & (2^TLC - 1)
         static_assert(F0::NR % (1 << TLC) == 0, "first-pass stride is whole tiles");
@@ -561,15 +578,15 @@ __device__ __forceinline__ void row_pass_body(const RowArgs& a) {
       }
     }
     if constexpr (iter && rho_in_buf) {
-      rfft<N, 0, true, LD>(v0, v, buf, tw, cb, [&]() {
+      rfft<G, 0, true, LD>(v0, v, buf, tw, cb, [&]() {
         __syncthreads();   // every thread's last read of the lines is done
         stage_rho();
         cp_commit();
       });
     } else if (iter || a.inv) {
-      rfft<N, 0, true, LD>(v0, v, buf, tw, cb);
+      rfft<G, 0, true, LD>(v0, v, buf, tw, cb);
     } else {
-      rfft<N, 0, false, LD>(v0, v, buf, tw, cb);
+      rfft<G, 0, false, LD>(v0, v, buf, tw, cb);
     }
   }
   float2* out = a.out + (long long)blockIdx.y * a.out_stride;
@@ -578,7 +595,7 @@ __device__ __forceinline__ void row_pass_body(const RowArgs& a) {
 #pragma unroll
     for (int b = 0; b < FL::B; ++b) {
       int l, j;
-      if (!bfly_of<N, FL::R>(b, cb, l, j)) continue;
+      if (!bfly_of<G, FL::R>(b, cb, l, j)) continue;
       if (l >= nrows) continue;
 #pragma unroll
       for (int r = 0; r < FL::R; ++r) {
@@ -595,7 +612,7 @@ __device__ __forceinline__ void row_pass_body(const RowArgs& a) {
 #pragma unroll
     for (int b = 0; b < FL::B; ++b) {
       int l, j;
-      if (!bfly_of<N, FL::R>(b, cb, l, j)) continue;
+      if (!bfly_of<G, FL::R>(b, cb, l, j)) continue;
       const uint4* m4 = reinterpret_cast<const uint4*>(mask_s + l * WPR + (j >> 5) * FL::R);
       uint4 mq = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
@@ -619,11 +636,11 @@ __device__ __forceinline__ void row_pass_body(const RowArgs& a) {
     }
     float2 o[IL::B][IL::R];
     if constexpr (rho_in_buf) __syncthreads();   // the rho rows are read before the lines are reused
-    rfft<N, 1, false, LD>(v, o, buf, tw, cb);
+    rfft<G, 1, false, LD>(v, o, buf, tw, cb);
 #pragma unroll
     for (int b = 0; b < IL::B; ++b) {
       int l, j;
-      if (!bfly_of<N, IL::R>(b, cb, l, j)) continue;
+      if (!bfly_of<G, IL::R>(b, cb, l, j)) continue;
       if (l >= nrows) continue;
       if constexpr (CT) {
         static_assert(IL::NS % (1 << TLC) == 0, "last-pass stride is whole tiles");
@@ -645,17 +662,17 @@ __device__ __forceinline__ void row_pass_body(const RowArgs& a) {
 
 // One kernel per update (ALGO is ignored in ROW_FFT mode): the executed code
 // holds a single update and no switch.
-template <int N, int MODE, int ALGO, bool SQ = false>
-__global__ void __launch_bounds__(Geom<N>::T, RGeom<N>::MINB_ROW) row_pass_rk(RowArgs a) {
+template <class G, int MODE, int ALGO, bool SQ = false>
+__global__ void __launch_bounds__(G::T, MODE == ROW_FFT ? RGeom<G>::MINB_ROW_FFT : RGeom<G>::MINB_ROW) row_pass_rk(RowArgs a) {
   pdl_wait_and_release();
   if (a.state && (a.state[blockIdx.y].flags & 4)) return;   // frozen pattern
-  row_pass_body<N, MODE, ALGO, SQ>(a);
+  row_pass_body<G, MODE, ALGO, SQ>(a);
 }
 // the compile-time layout of row_pass_rk<..., true> applies to these arguments
-template <int N>
+template <class G>
 __host__ __forceinline__ bool row_sq_layout(const RowArgs& a) {
-  constexpr int cbd = row_cb_pick(Geom<N>::LOG2L, rfft_cb_max<N>());
-  return row_sq_ok<N>() && a.mode == ROW_ITER && a.in_tiled && a.out_tiled && a.tile_log2 == Geom<N>::LOG2L && a.scale == 1.f &&
+  constexpr int cbd = row_cb_pick(G::LOG2L, rfft_cb_max<G::N>());
+  return row_sq_ok_g<G>() && a.mode == ROW_ITER && a.in_tiled && a.out_tiled && a.tile_log2 == G::LOG2L && a.scale == 1.f &&
          (a.cb_plus1 == 0 || a.cb_plus1 - 1 == cbd);
 }
 

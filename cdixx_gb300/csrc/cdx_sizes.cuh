@@ -37,34 +37,39 @@ template <int N>
 cudaError_t prepare_rk() {
   using G = Geom<N>;
   cudaError_t e;
-  if ((e = cudaFuncSetAttribute(row_pass_rk<N, ROW_FFT, ALGO_ER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                RGeom<N>::SMEM_ROW_LINES)) != cudaSuccess)
+  if ((e = cudaFuncSetAttribute(row_pass_rk<G, ROW_FFT, ALGO_ER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                RGeom<G>::SMEM_ROW_LINES)) != cudaSuccess)
     return e;
   const void* iter_kernels[] = {
-      (const void*)row_pass_rk<N, ROW_ITER, ALGO_HIO>, (const void*)row_pass_rk<N, ROW_ITER, ALGO_RAAR>,
-      (const void*)row_pass_rk<N, ROW_ITER, ALGO_ER>, (const void*)row_pass_rk<N, ROW_ITER, ALGO_POSER>,
-      (const void*)row_pass_rk<N, ROW_ITER, ALGO_POSHIO>, (const void*)row_pass_rk<N, ROW_ITER, ALGO_FHIO>};
+      (const void*)row_pass_rk<G, ROW_ITER, ALGO_HIO>, (const void*)row_pass_rk<G, ROW_ITER, ALGO_RAAR>,
+      (const void*)row_pass_rk<G, ROW_ITER, ALGO_ER>, (const void*)row_pass_rk<G, ROW_ITER, ALGO_POSER>,
+      (const void*)row_pass_rk<G, ROW_ITER, ALGO_POSHIO>, (const void*)row_pass_rk<G, ROW_ITER, ALGO_FHIO>};
   for (const void* k : iter_kernels)
-    if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, RGeom<N>::SMEM_ROW_ITER)) !=
+    if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, RGeom<G>::SMEM_ROW_ITER)) !=
         cudaSuccess)
       return e;
   if constexpr (row_sq_ok<N>()) {
     const void* sq_kernels[] = {
-        (const void*)row_pass_rk<N, ROW_ITER, ALGO_HIO, true>, (const void*)row_pass_rk<N, ROW_ITER, ALGO_RAAR, true>,
-        (const void*)row_pass_rk<N, ROW_ITER, ALGO_ER, true>, (const void*)row_pass_rk<N, ROW_ITER, ALGO_POSER, true>,
-        (const void*)row_pass_rk<N, ROW_ITER, ALGO_POSHIO, true>, (const void*)row_pass_rk<N, ROW_ITER, ALGO_FHIO, true>};
+        (const void*)row_pass_rk<G, ROW_ITER, ALGO_HIO, true>, (const void*)row_pass_rk<G, ROW_ITER, ALGO_RAAR, true>,
+        (const void*)row_pass_rk<G, ROW_ITER, ALGO_ER, true>, (const void*)row_pass_rk<G, ROW_ITER, ALGO_POSER, true>,
+        (const void*)row_pass_rk<G, ROW_ITER, ALGO_POSHIO, true>, (const void*)row_pass_rk<G, ROW_ITER, ALGO_FHIO, true>};
     for (const void* k : sq_kernels)
-      if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, RGeom<N>::SMEM_ROW_ITER)) !=
+      if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, RGeom<G>::SMEM_ROW_ITER)) !=
           cudaSuccess)
         return e;
   }
-  if ((e = cudaFuncSetAttribute(col_pass_rk<N, COL_FFT, PROJ_MODABS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  if ((e = cudaFuncSetAttribute(col_pass_rk<G, COL_FFT, PROJ_MODABS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 G::SMEM_LINES)) != cudaSuccess)
     return e;
-  if ((e = cudaFuncSetAttribute(col_pass_rk<N, COL_ITER, PROJ_MODABS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  if constexpr (WideGeom<N>::L != G::L) {
+    if ((e = cudaFuncSetAttribute(col_pass_rk<WideGeom<N>, COL_FFT, PROJ_MODABS, G::LOG2L>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize, WideGeom<N>::SMEM_LINES)) != cudaSuccess)
+      return e;
+  }
+  if ((e = cudaFuncSetAttribute(col_pass_rk<G, COL_ITER, PROJ_MODABS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 G::SMEM_COL_ITER)) != cudaSuccess)
     return e;
-  return cudaFuncSetAttribute(col_pass_rk<N, COL_ITER, PROJ_CCD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  return cudaFuncSetAttribute(col_pass_rk<G, COL_ITER, PROJ_CCD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               G::SMEM_COL_CCD);
 }
 
@@ -97,23 +102,23 @@ cudaError_t launch_row(const RowArgs& a, int batch, cudaStream_t st) {
     if (a.mode == ROW_ITER) row_pass_kernel<N, ROW_ITER, 1><<<grid, G::T, G::SMEM_ROW_ITER, st>>>(a);
     else row_pass_kernel<N, ROW_FFT, 1><<<grid, G::T, G::SMEM_LINES, st>>>(a);
   } else {
-    constexpr int SM = RGeom<N>::SMEM_ROW_ITER;
-    if (a.mode != ROW_ITER) return launch_pdl(row_pass_rk<N, ROW_FFT, ALGO_ER>, grid, G::T, RGeom<N>::SMEM_ROW_LINES, st, a, pdl_of<N>(a.pdl_mode));
-    if constexpr (row_sq_ok<N>()) if (row_sq_layout<N>(a)) switch (a.algo) {   // the compile-time layout of square patterns
-      case ALGO_HIO: return launch_pdl(row_pass_rk<N, ROW_ITER, ALGO_HIO, true>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
-      case ALGO_RAAR: return launch_pdl(row_pass_rk<N, ROW_ITER, ALGO_RAAR, true>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
-      case ALGO_ER: return launch_pdl(row_pass_rk<N, ROW_ITER, ALGO_ER, true>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
-      case ALGO_POSER: return launch_pdl(row_pass_rk<N, ROW_ITER, ALGO_POSER, true>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
-      case ALGO_POSHIO: return launch_pdl(row_pass_rk<N, ROW_ITER, ALGO_POSHIO, true>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
-      default: return launch_pdl(row_pass_rk<N, ROW_ITER, ALGO_FHIO, true>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
+    constexpr int SM = RGeom<G>::SMEM_ROW_ITER;
+    if (a.mode != ROW_ITER) return launch_pdl(row_pass_rk<G, ROW_FFT, ALGO_ER>, grid, G::T, RGeom<G>::SMEM_ROW_LINES, st, a, pdl_of<N>(a.pdl_mode));
+    if constexpr (row_sq_ok<N>()) if (row_sq_layout<G>(a)) switch (a.algo) {   // the compile-time layout of square patterns
+      case ALGO_HIO: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_HIO, true>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
+      case ALGO_RAAR: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_RAAR, true>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
+      case ALGO_ER: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_ER, true>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
+      case ALGO_POSER: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_POSER, true>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
+      case ALGO_POSHIO: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_POSHIO, true>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
+      default: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_FHIO, true>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
     }
     switch (a.algo) {   // unknown codes take the FHIO branch, as applySupport does (cdi.cc:25-36)
-      case ALGO_HIO: return launch_pdl(row_pass_rk<N, ROW_ITER, ALGO_HIO>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
-      case ALGO_RAAR: return launch_pdl(row_pass_rk<N, ROW_ITER, ALGO_RAAR>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
-      case ALGO_ER: return launch_pdl(row_pass_rk<N, ROW_ITER, ALGO_ER>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
-      case ALGO_POSER: return launch_pdl(row_pass_rk<N, ROW_ITER, ALGO_POSER>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
-      case ALGO_POSHIO: return launch_pdl(row_pass_rk<N, ROW_ITER, ALGO_POSHIO>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
-      default: return launch_pdl(row_pass_rk<N, ROW_ITER, ALGO_FHIO>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
+      case ALGO_HIO: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_HIO>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
+      case ALGO_RAAR: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_RAAR>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
+      case ALGO_ER: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_ER>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
+      case ALGO_POSER: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_POSER>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
+      case ALGO_POSHIO: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_POSHIO>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
+      default: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_FHIO>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
     }
   }
   return cudaGetLastError();
@@ -132,9 +137,17 @@ cudaError_t launch_col(const ColArgs& a, int batch, cudaStream_t st) {
     if (a.mode == COL_ITER) col_pass_kernel<N, COL_ITER, 1><<<grid, G::T, smem_iter, st>>>(a);
     else col_pass_kernel<N, COL_FFT, 1><<<grid, G::T, G::SMEM_LINES, st>>>(a);
   } else {
-    if (a.mode != COL_ITER) return launch_pdl(col_pass_rk<N, COL_FFT, PROJ_MODABS>, grid, G::T, G::SMEM_LINES, st, a, pdl_of<N>(a.pdl_mode));
-    if (a.proj == PROJ_CCD) return launch_pdl(col_pass_rk<N, COL_ITER, PROJ_CCD>, grid, G::T, smem_iter, st, a, pdl_of<N>(a.pdl_mode));
-    return launch_pdl(col_pass_rk<N, COL_ITER, PROJ_MODABS>, grid, G::T, smem_iter, st, a, pdl_of<N>(a.pdl_mode));
+    if constexpr (WideGeom<N>::L != G::L) {
+      // row-major data, and enough columns to give every SM a wide CTA
+      using W = WideGeom<N>;
+      if (a.mode != COL_ITER && !a.out_tiled &&
+          (long long)((a.cols + W::L - 1) / W::L) * batch >= sm_count())
+        return launch_pdl(col_pass_rk<W, COL_FFT, PROJ_MODABS, G::LOG2L>, dim3((a.cols + W::L - 1) / W::L, batch), W::T,
+                          W::SMEM_LINES, st, a, pdl_of<N>(a.pdl_mode));
+    }
+    if (a.mode != COL_ITER) return launch_pdl(col_pass_rk<G, COL_FFT, PROJ_MODABS>, grid, G::T, G::SMEM_LINES, st, a, pdl_of<N>(a.pdl_mode));
+    if (a.proj == PROJ_CCD) return launch_pdl(col_pass_rk<G, COL_ITER, PROJ_CCD>, grid, G::T, smem_iter, st, a, pdl_of<N>(a.pdl_mode));
+    return launch_pdl(col_pass_rk<G, COL_ITER, PROJ_MODABS>, grid, G::T, smem_iter, st, a, pdl_of<N>(a.pdl_mode));
   }
   return cudaGetLastError();
 }
