@@ -450,9 +450,14 @@ cudaError_t pattern_amp_sum(const float* amp, long long npx, int batch, double* 
   k_finalize_sum<<<batch, 32, 0, st>>>(part, nblk, stt, 0, 0.0, -1, 0, 0.f);
   return cudaGetLastError();
 }
-cudaError_t residual_rfactor(const float2* psi, const float* inten, long long npx, int batch, double* part, int nblk,
+// CTAs per pattern: 4096 pixels each, at most `most`; by the pattern's size alone, so a
+// pattern's sums are the same in any batch.  A CTA's two block sums cost as much as a few
+// thousand pixels (152 CTAs per pattern whatever its size: 458 us for 96 patterns of
+// 192^2, now about 60).
+cudaError_t residual_rfactor(const float2* psi, const float* inten, long long npx, int batch, double* part, int most,
                              PatState* stt, cudaStream_t st) {
   if (npx % 2) return cudaErrorInvalidValue;
+  const int nblk = (int)std::min<long long>(most, (npx + 4095) / 4096);
   k_res_rdiff<<<dim3(nblk, batch), kResThreads, 0, st>>>(psi, inten, npx, part, nblk);
   k_res_rdiff_finalize<<<batch, 32, 0, st>>>(part, nblk, stt);
   return cudaGetLastError();
