@@ -95,6 +95,7 @@ struct cdx_ctx {
   float2 *rho = nullptr, *work = nullptr, *psi = nullptr, *tmp = nullptr;
   float *inten = nullptr, *amp_t = nullptr, *inten_t = nullptr, *spt = nullptr, *bs = nullptr, *bs_t = nullptr;
   int tl = 0;              // log2 of the column-pass lines per CTA
+  int thin = 0;            // the passes' geometry for small work (use_thin)
   int cp = 0;              // cols padded to a multiple of 2^tl
   long long wstride = 0;   // rows * cp
   uint32_t* mask = nullptr;
@@ -285,6 +286,7 @@ int col_iter(cdx_ctx* c, bool from_psi, bool rf, float2* psi_proj = nullptr) {
   a.ccd_rcolor = (float)c->p.rcolor;
   a.pdl_mode = c->tune_pdl_col;
   a.err = c->derr;
+  a.thin = c->thin;
   CDX_CK(col_launcher(c->rows)(a, c->batch, c->st));
   return CDX_OK;
 }
@@ -312,9 +314,14 @@ int row_iter(cdx_ctx* c, int algo) {
   a.cb_plus1 = c->tune_cb_plus1;
   a.pdl_mode = c->tune_pdl_row;
   a.err = c->derr;
+  a.thin = c->thin;
   CDX_CK(row_launcher(c->cols)(a, c->batch, c->st));
   return CDX_OK;
 }
+
+// Whether the passes of `batch` rows x cols patterns take the geometry for small work
+// (cdx_rfft.cuh): up to 2^21 pixels a length of 1024 leaves SMs idle otherwise.
+bool use_thin(int rows, int cols, int batch) { return (long long)rows * cols * batch <= 1LL << 21; }
 
 // Generic 2-D transform of `batch` row-major patterns: rows then columns.
 int fft2_enqueue(const float2* in, float2* out, int rows, int cols, int batch, bool inv, float scale,
@@ -330,6 +337,7 @@ int fft2_enqueue(const float2* in, float2* out, int rows, int cols, int batch, b
   r.inv = inv;
   r.tc = tc;
   r.scale = 1.f;
+  r.thin = use_thin(rows, cols, batch);
   CDX_CK(row_launcher(cols)(r, batch, st));
   ColArgs c{};
   c.in = out;
@@ -341,6 +349,7 @@ int fft2_enqueue(const float2* in, float2* out, int rows, int cols, int batch, b
   c.inv = inv;
   c.tc = tc;
   c.scale = scale;
+  c.thin = r.thin;
   CDX_CK(col_launcher(rows)(c, batch, st));
   return CDX_OK;
 }
@@ -425,6 +434,7 @@ int enqueue_run(cdx_ctx* c, const std::vector<int>& steps, const SwPlan& sw, boo
     a.inv = 0;
     a.tc = c->p.fft_mode;
     a.scale = 1.f;
+    a.thin = c->thin;
     CDX_CK(col_launcher(c->rows)(a, c->batch, c->st));
     ++nl;
   }
@@ -911,7 +921,8 @@ int cdx_create(const cdx_params* p, void* stream, cdx_ctx** out) {
   if (prep_launcher(c->rows)() != cudaSuccess || prep_launcher(c->cols)() != cudaSuccess || misc_prepare() != cudaSuccess)
     return fail(set_error(CDX_ERR_CUDA, std::string("kernel attributes: ") + cudaGetErrorString(cudaGetLastError())));
   if ((e = twiddles(c->rows, &c->tw_r)) || (e = twiddles(c->cols, &c->tw_c))) return fail(e);
-  const int lc = lines_per_cta(c->rows);
+  c->thin = use_thin(c->rows, c->cols, c->batch);
+  const int lc = lines_per_cta(c->rows, c->thin, p->fft_mode != CDX_FFT_FP32);
   c->tl = 0;
   while ((1 << c->tl) < lc) ++c->tl;
   c->cp = (c->cols + lc - 1) / lc * lc;

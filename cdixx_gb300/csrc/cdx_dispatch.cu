@@ -20,7 +20,7 @@ template <int N> cudaError_t launch_col(const ColArgs&, int, cudaStream_t);
 #define CASE_PREP(N) case N: return &prepare_len<N>;
 #define CASE_ROW(N) case N: return &launch_row<N>;
 #define CASE_COL(N) case N: return &launch_col<N>;
-#define CASE_L(N) case N: return Geom<N>::L;
+#define CASE_L(N) case N: return tc ? Geom<N>::L : thin ? ThinGeom<N>::L : FGeom<N>::L;
 #define CASE_TW(N) case N: return Geom<N>::TWN;
 
 PrepLaunch prep_launcher(int n) {
@@ -32,7 +32,7 @@ RowLaunch row_launcher(int n) {
 ColLaunch col_launcher(int n) {
   switch (n) { CDX_FOR_EACH_SIZE(CASE_COL) default: return nullptr; }
 }
-int lines_per_cta(int n) {
+int lines_per_cta(int n, bool thin, bool tc) {
   switch (n) { CDX_FOR_EACH_SIZE(CASE_L) default: return 0; }
 }
 int twiddle_count(int n) {

@@ -293,7 +293,8 @@ struct GeomT {
   static constexpr int SMEM_MAX = SMEM_ROW_ITER > SMEM_COL_CCD ? SMEM_ROW_ITER : SMEM_COL_CCD;
   __device__ __forceinline__ static int idx(int l, int i) { return l * LD + i + (i >> 4); }
 };
-// The geometry of length N: tiles of L columns have a power-of-two width and a
+// The geometry of length N in the tensor-core modes (the FP32 passes have their own,
+// FGeom in cdx_rfft.cuh): tiles of L columns have a power-of-two width and a
 // row CTA moves at least 32-byte pieces of them; small CTAs keep three or more
 // resident per SM (512 threads at 3072 and 4096).
 constexpr int geom_t(int n) { return n >= 3072 ? 512 : 256; }

@@ -72,7 +72,7 @@ struct PtyKernels {
 };
 #define PTY_CASE(N) \
   case N: k.prep = &pty_prepare<N>; k.fwd = &pty_launch_fwd<N>; k.upd = &pty_launch_upd<N>; \
-          k.col = &pty_launch_col<N>; k.L = Geom<N>::L; return true;
+          k.col = &pty_launch_col<N>; k.L = FGeom<N>::L; return true;
 bool pty_kernels(int n, PtyKernels& k) {
   switch (n) {
     PTY_CASE(16) PTY_CASE(24) PTY_CASE(32) PTY_CASE(48) PTY_CASE(64) PTY_CASE(96) PTY_CASE(128)

@@ -113,15 +113,16 @@ __device__ __forceinline__ long long pty_tiled(int r, int c, int rows, int tl) {
 template <int N>
 struct PtyRow {
   static constexpr int SN = N + 8;
-  static constexpr int STAGE = 2 * Geom<N>::L * SN * (int)sizeof(float2);
-  static constexpr int LD = RGeom<Geom<N>>::ROW_LD;
-  static constexpr int SMEM = RGeom<Geom<N>>::SMEM_ROW_LINES + STAGE;
+  static constexpr int MINB = FGeom<N>::T >= 512 ? 1 : (FGeom<N>::T < 256 ? 512 : 768) / FGeom<N>::T;
+  static constexpr int STAGE = 2 * FGeom<N>::L * SN * (int)sizeof(float2);
+  static constexpr int LD = RGeom<FGeom<N>>::ROW_LD;
+  static constexpr int SMEM = RGeom<FGeom<N>>::SMEM_ROW_LINES + STAGE;
 };
 
 template <int N>
 __device__ __forceinline__ void pty_stage_rows(const PtyArgs& a, float2* o_s, float2* p_s, int row0, int nrows,
                                                int2 w) {
-  using G = Geom<N>;
+  using G = FGeom<N>;
   constexpr int L = G::L, T = G::T, SN = PtyRow<N>::SN;
   const long long OC = a.obj_cols;
   for (int e = threadIdx.x; e < L * N; e += T) {
@@ -139,8 +140,8 @@ __device__ __forceinline__ void pty_stage_rows(const PtyArgs& a, float2* o_s, fl
 // ------------------------------------------------------- forward row pass
 // FRES: isFresnel, a separate instantiation so the plain kernels carry no phase code
 template <int N, bool FRES>
-__global__ void __launch_bounds__(Geom<N>::T, Geom<N>::MINB) pty_fwd_rk(PtyArgs a) {
-  using G = Geom<N>;
+__global__ void __launch_bounds__(FGeom<N>::T, PtyRow<N>::MINB) pty_fwd_rk(PtyArgs a) {
+  using G = FGeom<N>;
   constexpr int L = G::L;
   using F0 = RFirst<G, 0>;
   using FL = RLast<G, 0>;
@@ -181,8 +182,8 @@ __global__ void __launch_bounds__(Geom<N>::T, Geom<N>::MINB) pty_fwd_rk(PtyArgs 
 
 // ------------------------------------------------------------ column pass
 template <int N>
-__global__ void __launch_bounds__(Geom<N>::T, RGeom<Geom<N>>::MINB_COL) pty_col_rk(PtyArgs a) {
-  using G = Geom<N>;
+__global__ void __launch_bounds__(FGeom<N>::T, RGeom<FGeom<N>>::MINB_COL) pty_col_rk(PtyArgs a) {
+  using G = FGeom<N>;
   constexpr int L = G::L, T = G::T;
   using F0 = RFirst<G, 0>;
   using FL = RLast<G, 0>;
@@ -256,8 +257,8 @@ __global__ void __launch_bounds__(Geom<N>::T, RGeom<Geom<N>>::MINB_COL) pty_col_
 
 // -------------------------------------------------------- update row pass
 template <int N, bool FRES>
-__global__ void __launch_bounds__(Geom<N>::T, Geom<N>::MINB) pty_upd_rk(PtyArgs a) {
-  using G = Geom<N>;
+__global__ void __launch_bounds__(FGeom<N>::T, PtyRow<N>::MINB) pty_upd_rk(PtyArgs a) {
+  using G = FGeom<N>;
   constexpr int L = G::L;
   using F0 = RFirst<G, 0>;
   using FL = RLast<G, 0>;
@@ -323,7 +324,7 @@ __global__ void __launch_bounds__(Geom<N>::T, Geom<N>::MINB) pty_upd_rk(PtyArgs 
 // Launchers of the three kernels for line length N (host side).
 template <int N>
 cudaError_t pty_prepare() {
-  using G = Geom<N>;
+  using G = FGeom<N>;
   cudaError_t e = cudaSuccess;
   const void* rows_k[] = {(const void*)pty_fwd_rk<N, false>, (const void*)pty_fwd_rk<N, true>,
                           (const void*)pty_upd_rk<N, false>, (const void*)pty_upd_rk<N, true>};
@@ -336,21 +337,21 @@ cudaError_t pty_prepare() {
 }
 template <int N>
 cudaError_t pty_launch_fwd(const PtyArgs& a, cudaStream_t st) {
-  using G = Geom<N>;
+  using G = FGeom<N>;
   const dim3 grid((a.rows + G::L - 1) / G::L);
   return a.fresnel != 0.f ? launch_pdl(pty_fwd_rk<N, true>, grid, G::T, PtyRow<N>::SMEM, st, a)
                           : launch_pdl(pty_fwd_rk<N, false>, grid, G::T, PtyRow<N>::SMEM, st, a);
 }
 template <int N>
 cudaError_t pty_launch_upd(const PtyArgs& a, cudaStream_t st) {
-  using G = Geom<N>;
+  using G = FGeom<N>;
   const dim3 grid((a.rows + G::L - 1) / G::L);
   return a.fresnel != 0.f ? launch_pdl(pty_upd_rk<N, true>, grid, G::T, PtyRow<N>::SMEM, st, a)
                           : launch_pdl(pty_upd_rk<N, false>, grid, G::T, PtyRow<N>::SMEM, st, a);
 }
 template <int N>
 cudaError_t pty_launch_col(const PtyArgs& a, cudaStream_t st) {
-  using G = Geom<N>;
+  using G = FGeom<N>;
   return launch_pdl(pty_col_rk<N>, dim3((a.cols + G::L - 1) / G::L), G::T,
                     G::SMEM_LINES + 2 * G::L * N * (int)sizeof(float), st, a);
 }

@@ -216,21 +216,41 @@ __device__ __forceinline__ void rfft(float2 (&in)[RFirst<G, PLAN>::B][RFirst<G, 
   }
 }
 
-// Shared memory and resident CTAs per SM (register budget) of the
-// register-handoff kernels.  The column pass at 256 threads is budgeted for 4
-// CTAs per SM (64 registers, no spills; 2-4 % faster than 3).  The row pass
-// stages its rho rows in the line buffer (loading rho straight from global
-// memory instead was 4-30 % slower, its latency exposed) and is budgeted for 4
-// CTAs per SM below 1024 and 3 from 1024 up, where the radix-16 last passes
-// would spill at 64 registers (2048^2: 80 registers, 50.5 -> 49.7 us per
-// iteration; 512^2 x16 is faster at 4).
-#ifndef CDX_RK_MINB_COL
-#define CDX_RK_MINB_COL 4
-#endif
+// FP32 launch geometry per length: threads of a CTA (its lines hold about 16 values
+// per thread) and the threads per SM its register budget leaves room for.  Small
+// CTAs spread a small pattern over more SMs and leave shorter tails; the registers
+// (64 a thread at 1024 threads per SM, 80 at 768) trade occupancy for spills.
+// Measured, us per iteration, against 256 threads (the geometry of the tensor-core
+// modes) at its best budget, L2 warm:
+//   64^2 (64 threads)   x1 12.9 -> 10.9, x300 16.7 -> 16.3
+//   128^2 (64)          x1 12.2 -> 8.7, x30 13.0 -> 10.5, x100 25.2 -> 17.3, x200 37.3 -> 29.5
+//   192^2 (64)          x1 12.6 -> 9.2, x8 13.2 -> 10.3, x96 46.8 -> 42.5
+//   256^2 (128)         x1 11.1 -> 9.1, x16 15.1 -> 13.8, x64 39.4 -> 35.5
+//   512^2 (128)         x1 11.9 -> 10.5, x16 44.5 -> 43.1, x48 144.3 -> 138.8
+//   768^2 (192)         x1 16.4 -> 14.7, x2 23.5 -> 21.7, x8 59.8 -> 54.8
+// (1536 on 192: square x1 43.2 -> 42.3, but 768 x 1536 25.0 -> 31.1, so it stays at 256.)
+// 192 threads at 768 keep every thread busy in the radix-16 passes.  384
+// stays at 256 (96 threads: x1 12.7 -> 12.3 but x8 22.2 -> 23.1, x47 82.6 -> 85.2), as
+// do 96 (96 threads: x1 13.3 -> 14.4) and 1024 (128 threads: x4 48.4 -> 50.1) but for
+// small work: up to 2^21 pixels a 1024 pass runs on 128 threads with 128 registers
+// (1024^2 x1 24.2 -> 17.7, x2 29.4 -> 28.3; use_thin).
+constexpr int fp_t(int n) {
+  return n == 64 || n == 128 || n == 192 ? 64 : n == 256 || n == 512 ? 128 : n == 768 ? 192 : geom_t(n);
+}
+constexpr int lines_of(int n, int t) { return pow2_floor(16 * t / n < 2 ? 2 : 16 * t / n); }
+template <int N>
+struct FGeom : GeomT<N, fp_t(N), lines_of(N, fp_t(N))> {};
+constexpr int thin_t(int n) { return n == 1024 ? 128 : fp_t(n); }
+template <int N>
+struct ThinGeom : GeomT<N, thin_t(N), lines_of(N, thin_t(N))> {};
+// threads per SM of the register budget (512 threads and more: two CTAs of 512, else one)
+constexpr int res_col(int n, int t) {
+  return t >= 512 ? (t == 512 ? 1024 : t) : n == 1024 && t == 128 ? 512 : n == 128 || n == 192 || t == 192 ? 768 : 1024;
+}
+constexpr int res_row(int n, int t) { return t >= 512 ? t : n >= 1024 && t == 256 ? 768 : res_col(n, t); }
 
-#ifndef CDX_RK_MINB_ROW
-#define CDX_RK_MINB_ROW 0
-#endif
+// The row pass stages its rho rows in the line buffer (loading rho straight from
+// global memory instead was 4-30 % slower, its latency exposed).
 // RHO_IN_BUF: the iterating row pass stages its rho rows in the FFT line buffer
 // itself, copied in after the inverse transform's last shared-memory read (the
 // copy overlaps the last pass's arithmetic), so the CTA needs one line buffer
@@ -241,13 +261,11 @@ __device__ __forceinline__ void rfft(float2 (&in)[RFirst<G, PLAN>::B][RFirst<G, 
 template <class G>
 struct RGeom {
   static constexpr int N = G::N;
-  static constexpr bool RHO_IN_BUF = CDX_RHO_IN_BUF && G::T == 256 && plan_len(N) > 1;
+  static constexpr bool RHO_IN_BUF = CDX_RHO_IN_BUF && G::T <= 256 && plan_len(N) > 1;
   static constexpr int ROW_LD = row_line_stride<G>();
   static constexpr int SMEM_ROW_LINES = G::L * ROW_LD * (int)sizeof(float2);
   static constexpr int SMEM_ROW_ITER = SMEM_ROW_LINES * (RHO_IN_BUF ? 1 : 2) + G::L * ((N + 31) >> 5) * 4;
-  static constexpr int MINB_COL = (CDX_RK_MINB_COL > 0 && G::T == 256) ? CDX_RK_MINB_COL : (G::T == 512 ? 2 : 1);
-  static constexpr int MINB_ROW =
-      (CDX_RK_MINB_ROW > 0 && G::T == 256) ? CDX_RK_MINB_ROW : (RHO_IN_BUF ? (N >= 1024 ? 3 : 4) : G::MINB);
+  static constexpr int MINB_COL = res_col(N, G::T) / G::T, MINB_ROW = res_row(N, G::T) / G::T;
   static constexpr int MINB_ROW_FFT = G::T == 512 ? 2 : MINB_ROW;
 };
 // Geometry of a column transform alone whose output is row-major: the default
@@ -257,9 +275,9 @@ struct RGeom {
 // 3072^2 123 -> 95, 2048^2 46.0 -> 37.0, 1024^2 x8 61.7 -> 57.4; 4 columns at 2048^2
 // 39.5; 8 at 768^2 x8 35.4 -> 38.3, so 768 keeps its own).  Two CTAs of 512 threads
 // per SM in the row transforms of 3072 and 4096 are part of it.
-constexpr int wide_l(int n) { return n >= 3072 ? 4 : (n >= 1024 ? 8 : geom_l(n)); }
+constexpr int wide_l(int n) { return n >= 3072 ? 4 : (n >= 1024 ? 8 : lines_of(n, fp_t(n))); }
 template <int N>
-struct WideGeom : GeomT<N, wide_l(N) == geom_l(N) ? geom_t(N) : wide_l(N) * N / 16, wide_l(N)> {};
+struct WideGeom : GeomT<N, wide_l(N) == FGeom<N>::L ? fp_t(N) : wide_l(N) * N / 16, wide_l(N)> {};
 
 // ------------------------------------------------------------- real-space updates
 template <int ALGO>

@@ -35,44 +35,41 @@ cudaError_t prepare_tc() {
   return e != cudaSuccess ? e : prepare_tc_mode<N, 2>();
 }
 
+template <class K>
+cudaError_t max_smem(K* kernel, int bytes) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+template <class G, bool SQ>
+cudaError_t prepare_row_g() {
+  constexpr int SM = RGeom<G>::SMEM_ROW_ITER;
+  cudaError_t e;
+  if ((e = max_smem(row_pass_rk<G, ROW_ITER, ALGO_HIO, SQ>, SM)) != cudaSuccess) return e;
+  if ((e = max_smem(row_pass_rk<G, ROW_ITER, ALGO_RAAR, SQ>, SM)) != cudaSuccess) return e;
+  if ((e = max_smem(row_pass_rk<G, ROW_ITER, ALGO_ER, SQ>, SM)) != cudaSuccess) return e;
+  if ((e = max_smem(row_pass_rk<G, ROW_ITER, ALGO_POSER, SQ>, SM)) != cudaSuccess) return e;
+  if ((e = max_smem(row_pass_rk<G, ROW_ITER, ALGO_POSHIO, SQ>, SM)) != cudaSuccess) return e;
+  return max_smem(row_pass_rk<G, ROW_ITER, ALGO_FHIO, SQ>, SM);
+}
+template <class G>
+cudaError_t prepare_g() {
+  cudaError_t e;
+  if ((e = max_smem(row_pass_rk<G, ROW_FFT, ALGO_ER>, RGeom<G>::SMEM_ROW_LINES)) != cudaSuccess) return e;
+  if ((e = prepare_row_g<G, false>()) != cudaSuccess) return e;
+  if constexpr (row_sq_ok_g<G>()) if ((e = prepare_row_g<G, true>()) != cudaSuccess) return e;
+  if ((e = max_smem(col_pass_rk<G, COL_FFT, PROJ_MODABS>, G::SMEM_LINES)) != cudaSuccess) return e;
+  if ((e = max_smem(col_pass_rk<G, COL_ITER, PROJ_MODABS>, G::SMEM_COL_ITER)) != cudaSuccess) return e;
+  return max_smem(col_pass_rk<G, COL_ITER, PROJ_CCD>, G::SMEM_COL_CCD);
+}
+
 template <int N>
 cudaError_t prepare_rk() {
-  using G = Geom<N>;
-  cudaError_t e;
-  if ((e = cudaFuncSetAttribute(row_pass_rk<G, ROW_FFT, ALGO_ER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                RGeom<G>::SMEM_ROW_LINES)) != cudaSuccess)
-    return e;
-  const void* iter_kernels[] = {
-      (const void*)row_pass_rk<G, ROW_ITER, ALGO_HIO>, (const void*)row_pass_rk<G, ROW_ITER, ALGO_RAAR>,
-      (const void*)row_pass_rk<G, ROW_ITER, ALGO_ER>, (const void*)row_pass_rk<G, ROW_ITER, ALGO_POSER>,
-      (const void*)row_pass_rk<G, ROW_ITER, ALGO_POSHIO>, (const void*)row_pass_rk<G, ROW_ITER, ALGO_FHIO>};
-  for (const void* k : iter_kernels)
-    if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, RGeom<G>::SMEM_ROW_ITER)) !=
-        cudaSuccess)
-      return e;
-  if constexpr (row_sq_ok<N>()) {
-    const void* sq_kernels[] = {
-        (const void*)row_pass_rk<G, ROW_ITER, ALGO_HIO, true>, (const void*)row_pass_rk<G, ROW_ITER, ALGO_RAAR, true>,
-        (const void*)row_pass_rk<G, ROW_ITER, ALGO_ER, true>, (const void*)row_pass_rk<G, ROW_ITER, ALGO_POSER, true>,
-        (const void*)row_pass_rk<G, ROW_ITER, ALGO_POSHIO, true>, (const void*)row_pass_rk<G, ROW_ITER, ALGO_FHIO, true>};
-    for (const void* k : sq_kernels)
-      if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, RGeom<G>::SMEM_ROW_ITER)) !=
-          cudaSuccess)
-        return e;
-  }
-  if ((e = cudaFuncSetAttribute(col_pass_rk<G, COL_FFT, PROJ_MODABS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                G::SMEM_LINES)) != cudaSuccess)
-    return e;
-  if constexpr (WideGeom<N>::L != G::L) {
-    if ((e = cudaFuncSetAttribute(col_pass_rk<WideGeom<N>, COL_FFT, PROJ_MODABS, G::LOG2L>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, WideGeom<N>::SMEM_LINES)) != cudaSuccess)
-      return e;
-  }
-  if ((e = cudaFuncSetAttribute(col_pass_rk<G, COL_ITER, PROJ_MODABS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                G::SMEM_COL_ITER)) != cudaSuccess)
-    return e;
-  return cudaFuncSetAttribute(col_pass_rk<G, COL_ITER, PROJ_CCD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              G::SMEM_COL_CCD);
+  using G = FGeom<N>;
+  using W = WideGeom<N>;
+  cudaError_t e = prepare_g<G>();
+  if constexpr (ThinGeom<N>::T != G::T) if (e == cudaSuccess) e = prepare_g<ThinGeom<N>>();
+  if constexpr (W::L != G::L)
+    if (e == cudaSuccess) e = max_smem(col_pass_rk<W, COL_FFT, PROJ_MODABS, G::LOG2L>, W::SMEM_LINES);
+  return e;
 }
 
 // Raise the dynamic shared-memory limit of the kernels of length N on the
@@ -101,6 +98,31 @@ constexpr bool pass_pdl() { return N != 2048; }
 template <int N>
 bool pdl_of(int mode) { return mode == 0 ? pass_pdl<N>() : mode == 2; }
 
+template <class G>
+cudaError_t launch_row_g(const RowArgs& a, int batch, cudaStream_t st) {
+  constexpr int N = G::N, SM = RGeom<G>::SMEM_ROW_ITER;
+  const dim3 grid((a.rows + G::L - 1) / G::L, batch);
+  const bool pdl = pdl_of<N>(a.pdl_mode);
+  if (a.mode != ROW_ITER)
+    return launch_pdl(row_pass_rk<G, ROW_FFT, ALGO_ER>, grid, G::T, RGeom<G>::SMEM_ROW_LINES, st, a, pdl);
+  if constexpr (row_sq_ok_g<G>()) if (row_sq_layout<G>(a)) switch (a.algo) {   // the compile-time layout of square patterns
+    case ALGO_HIO: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_HIO, true>, grid, G::T, SM, st, a, pdl);
+    case ALGO_RAAR: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_RAAR, true>, grid, G::T, SM, st, a, pdl);
+    case ALGO_ER: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_ER, true>, grid, G::T, SM, st, a, pdl);
+    case ALGO_POSER: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_POSER, true>, grid, G::T, SM, st, a, pdl);
+    case ALGO_POSHIO: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_POSHIO, true>, grid, G::T, SM, st, a, pdl);
+    default: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_FHIO, true>, grid, G::T, SM, st, a, pdl);
+  }
+  switch (a.algo) {   // unknown codes take the FHIO branch, as applySupport does (cdi.cc:25-36)
+    case ALGO_HIO: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_HIO>, grid, G::T, SM, st, a, pdl);
+    case ALGO_RAAR: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_RAAR>, grid, G::T, SM, st, a, pdl);
+    case ALGO_ER: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_ER>, grid, G::T, SM, st, a, pdl);
+    case ALGO_POSER: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_POSER>, grid, G::T, SM, st, a, pdl);
+    case ALGO_POSHIO: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_POSHIO>, grid, G::T, SM, st, a, pdl);
+    default: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_FHIO>, grid, G::T, SM, st, a, pdl);
+  }
+}
+
 template <int N>
 cudaError_t launch_row(const RowArgs& a, int batch, cudaStream_t st) {
   using G = Geom<N>;
@@ -113,26 +135,19 @@ cudaError_t launch_row(const RowArgs& a, int batch, cudaStream_t st) {
     if (a.mode == ROW_ITER) row_pass_kernel<N, ROW_ITER, 1><<<grid, G::T, G::SMEM_ROW_ITER, st>>>(a);
     else row_pass_kernel<N, ROW_FFT, 1><<<grid, G::T, G::SMEM_LINES, st>>>(a);
   } else {
-    constexpr int SM = RGeom<G>::SMEM_ROW_ITER;
-    if (a.mode != ROW_ITER) return launch_pdl(row_pass_rk<G, ROW_FFT, ALGO_ER>, grid, G::T, RGeom<G>::SMEM_ROW_LINES, st, a, pdl_of<N>(a.pdl_mode));
-    if constexpr (row_sq_ok<N>()) if (row_sq_layout<G>(a)) switch (a.algo) {   // the compile-time layout of square patterns
-      case ALGO_HIO: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_HIO, true>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
-      case ALGO_RAAR: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_RAAR, true>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
-      case ALGO_ER: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_ER, true>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
-      case ALGO_POSER: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_POSER, true>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
-      case ALGO_POSHIO: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_POSHIO, true>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
-      default: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_FHIO, true>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
-    }
-    switch (a.algo) {   // unknown codes take the FHIO branch, as applySupport does (cdi.cc:25-36)
-      case ALGO_HIO: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_HIO>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
-      case ALGO_RAAR: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_RAAR>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
-      case ALGO_ER: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_ER>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
-      case ALGO_POSER: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_POSER>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
-      case ALGO_POSHIO: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_POSHIO>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
-      default: return launch_pdl(row_pass_rk<G, ROW_ITER, ALGO_FHIO>, grid, G::T, SM, st, a, pdl_of<N>(a.pdl_mode));
-    }
+    if constexpr (ThinGeom<N>::T != FGeom<N>::T) if (a.thin) return launch_row_g<ThinGeom<N>>(a, batch, st);
+    return launch_row_g<FGeom<N>>(a, batch, st);
   }
   return cudaGetLastError();
+}
+
+template <class G>
+cudaError_t launch_col_g(const ColArgs& a, int batch, cudaStream_t st) {
+  const dim3 grid((a.cols + G::L - 1) / G::L, batch);
+  const bool pdl = pdl_of<G::N>(a.pdl_mode);
+  if (a.mode != COL_ITER) return launch_pdl(col_pass_rk<G, COL_FFT, PROJ_MODABS>, grid, G::T, G::SMEM_LINES, st, a, pdl);
+  if (a.proj == PROJ_CCD) return launch_pdl(col_pass_rk<G, COL_ITER, PROJ_CCD>, grid, G::T, G::SMEM_COL_CCD, st, a, pdl);
+  return launch_pdl(col_pass_rk<G, COL_ITER, PROJ_MODABS>, grid, G::T, G::SMEM_COL_ITER, st, a, pdl);
 }
 
 template <int N>
@@ -148,17 +163,17 @@ cudaError_t launch_col(const ColArgs& a, int batch, cudaStream_t st) {
     if (a.mode == COL_ITER) col_pass_kernel<N, COL_ITER, 1><<<grid, G::T, smem_iter, st>>>(a);
     else col_pass_kernel<N, COL_FFT, 1><<<grid, G::T, G::SMEM_LINES, st>>>(a);
   } else {
-    if constexpr (WideGeom<N>::L != G::L) {
-      // row-major data, and enough columns to give every SM a wide CTA
+    using F = FGeom<N>;
+    if constexpr (ThinGeom<N>::T != F::T) if (a.thin) return launch_col_g<ThinGeom<N>>(a, batch, st);
+    if constexpr (WideGeom<N>::L != F::L) {
+      // row-major output, and enough columns to give every SM a wide CTA
       using W = WideGeom<N>;
-      if (a.mode != COL_ITER && !a.out_tiled &&
-          (long long)((a.cols + W::L - 1) / W::L) * batch >= sm_count())
-        return launch_pdl(col_pass_rk<W, COL_FFT, PROJ_MODABS, G::LOG2L>, dim3((a.cols + W::L - 1) / W::L, batch), W::T,
-                          W::SMEM_LINES, st, a, pdl_of<N>(a.pdl_mode));
+      const int w = (a.cols + W::L - 1) / W::L;
+      if (a.mode != COL_ITER && !a.out_tiled && (long long)w * batch >= sm_count())
+        return launch_pdl(col_pass_rk<W, COL_FFT, PROJ_MODABS, F::LOG2L>, dim3(w, batch), W::T, W::SMEM_LINES, st, a,
+                          pdl_of<N>(a.pdl_mode));
     }
-    if (a.mode != COL_ITER) return launch_pdl(col_pass_rk<G, COL_FFT, PROJ_MODABS>, grid, G::T, G::SMEM_LINES, st, a, pdl_of<N>(a.pdl_mode));
-    if (a.proj == PROJ_CCD) return launch_pdl(col_pass_rk<G, COL_ITER, PROJ_CCD>, grid, G::T, smem_iter, st, a, pdl_of<N>(a.pdl_mode));
-    return launch_pdl(col_pass_rk<G, COL_ITER, PROJ_MODABS>, grid, G::T, smem_iter, st, a, pdl_of<N>(a.pdl_mode));
+    return launch_col_g<F>(a, batch, st);
   }
   return cudaGetLastError();
 }

@@ -71,6 +71,7 @@ struct RowArgs {
   int cb_plus1;            // 0: default butterfly chunk bits; k + 1: chunk bits k (autotuner)
   int pdl_mode;            // 0: the per-length default, 1: plain launch, 2: programmatic dependent launch
   int* err;                // optional: bit 0 set when a bulk copy's wait ran out
+  int thin;                // 1: the geometry for small work (lengths that have one)
 };
 
 struct ColArgs {
@@ -97,6 +98,7 @@ struct ColArgs {
   float ccd_rcolor;        // vars.rcolor
   int pdl_mode;            // as RowArgs::pdl_mode
   int* err;                // as RowArgs::err
+  int thin;                // as RowArgs::thin; column-tiled arrays then have that geometry's width
 };
 
 // Launch helpers exported by the per-size translation units.
@@ -107,7 +109,8 @@ typedef cudaError_t (*ColLaunch)(const ColArgs&, int batch, cudaStream_t);
 PrepLaunch prep_launcher(int n);   // nullptr: unsupported length
 RowLaunch row_launcher(int n);
 ColLaunch col_launcher(int n);
-int lines_per_cta(int n);          // lines (rows or columns) per CTA for length n
+// lines (rows or columns) per CTA for length n: the FP32 geometry, its thin one, or the tensor-core modes'
+int lines_per_cta(int n, bool thin = false, bool tc = false);
 int twiddle_count(int n);          // entries of the per-pass twiddle table of length n
 int row_cb_default(int n, int tile_log2);   // butterfly chunk bits the row pass uses on tiled data
 int row_cb_max(int n);                      // largest valid chunk bits of length n
