@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <type_traits>
 #include <cstring>
@@ -22,6 +23,7 @@
 #include "cdx_types.h"
 #include "cdx_unet.h"
 #include "cdx_unet_gemm.cuh"
+#include "cdx_unet_umma.cuh"
 
 namespace cdx {
 namespace unet {
@@ -64,9 +66,11 @@ __global__ void k_prep_input(const float* __restrict__ inten, const unsigned* __
 }
 
 // FP32 weights [co][kh][kw][ci] (real sizes) -> BF16 [co_p][kh][kw][ci_p] and
-// transposed [ci_p][kh][kw][co_p], zero-padded
+// transposed [ci_p][kh][kw][co_p], zero-padded, and both packed for k_conv_umma
+// ([K/8][columns][8], K = (kh, kw, ci) or (kh, kw, co))
 __global__ void k_weights_bf16(const float* __restrict__ w, int co_r, int ci_r, int co_p, int ci_p, int kk,
-                               __nv_bfloat16* __restrict__ wb, __nv_bfloat16* __restrict__ wt) {
+                               __nv_bfloat16* __restrict__ wb, __nv_bfloat16* __restrict__ wt,
+                               __nv_bfloat16* __restrict__ pb, __nv_bfloat16* __restrict__ pt) {
   const long long total = (long long)co_p * kk * ci_p;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const int ci = (int)(i % ci_p);
@@ -76,6 +80,9 @@ __global__ void k_weights_bf16(const float* __restrict__ w, int co_r, int ci_r, 
     const __nv_bfloat16 b = __float2bfloat16(v);
     wb[i] = b;
     wt[((long long)ci * kk + k) * co_p + co] = b;
+    const int kb = k * ci_p + ci, kt = k * co_p + co;
+    pb[((long long)(kb >> 3) * co_p + co) * 8 + (kb & 7)] = b;
+    pt[((long long)(kt >> 3) * ci_p + ci) * 8 + (kt & 7)] = b;
   }
 }
 
@@ -639,6 +646,7 @@ struct Layer {
   // convolution and (cin, cout) for a transposed one
   int wco_r, wci_r, wco_p, wci_p;
   __nv_bfloat16 *wb = nullptr, *wt = nullptr;
+  __nv_bfloat16 *pb = nullptr, *pt = nullptr;   // the same, packed for k_conv_umma
   int in0 = -1, in1 = -1;             // producer layers (-1: the network input)
   float* pre = nullptr;               // conv output (FP32)
   __nv_bfloat16* act = nullptr;       // activation (BF16)
@@ -745,7 +753,9 @@ int build(Net* u) {
   for (auto& l : u->L) {
     const size_t px = (size_t)B * l.out_h * l.out_h;
     const size_t wsz = (size_t)l.wco_p * l.k * l.k * l.wci_p;
-    if ((e = dalloc(u, &l.wb, wsz)) || (e = dalloc(u, &l.wt, wsz))) return e;
+    if ((e = dalloc(u, &l.wb, wsz)) || (e = dalloc(u, &l.wt, wsz)) || (e = dalloc(u, &l.pb, wsz)) ||
+        (e = dalloc(u, &l.pt, wsz)))
+      return e;
     if ((e = dalloc(u, &l.pre, px * l.cout_p)) || (e = dalloc(u, &l.act, px * l.cout_p)) ||
         (e = dalloc(u, &l.dact, px * l.cout_p)) || (e = dalloc(u, &l.dpre, px * l.cout_p)))
       return e;
@@ -795,7 +805,7 @@ int refresh_weights(Net* u) {
   for (auto& l : u->L) {
     const long long tot = (long long)l.wco_p * l.k * l.k * l.wci_p;
     k_weights_bf16<<<grid_for(tot), kThreads, 0, u->st>>>(u->params + l.w_off, l.wco_r, l.wci_r, l.wco_p, l.wci_p,
-                                                           l.k * l.k, l.wb, l.wt);
+                                                           l.k * l.k, l.wb, l.wt, l.pb, l.pt);
   }
   U_CK(cudaGetLastError());
   u->weights_dirty = false;
@@ -832,11 +842,50 @@ int launch_umma(const Op& op, long long M, int NC, int K, int* err, cudaStream_t
   return CDX_OK;
 }
 
-// forward (DGRAD false) or data-gradient GEMM: tcgen05 tiles when the net is
-// configured for them, else the mma.sync kernel
+// The convolution (or its data gradient) on k_conv_umma, where the layer fits it:
+// 3x3 and 2x2 layers of 16 to 256 channels in and out.
 template <bool DGRAD>
-int launch_gemm(const Net* u, const GemmArgs& a, cudaStream_t st) {
+bool plan_umma(const GemmArgs& g, const __nv_bfloat16* packed, ConvUmma& a, int& smem) {
+  const ConvShape& s = g.s;
+  a = ConvUmma{};
+  a.w = packed;
+  a.nimg = s.N;
+  a.acc0 = g.acc0;
+  a.acc1 = g.acc1;
+  a.out0 = g.out0;
+  const bool k3 = s.KH == 3 && s.KW == 3 && s.P == 1, k2 = s.KH == 2 && s.KW == 2 && s.P == 0;
+  if (!DGRAD) {
+    a.x0 = g.x0; a.x1 = g.x1; a.C0 = s.C0; a.C = s.Cin;
+    a.N = a.N0 = s.Cout;
+    a.out1 = g.out0;
+    a.H = s.H; a.W = s.W; a.GH = a.OH = s.Ho; a.GW = a.OW = s.Wo;
+    if (k3 && s.S == 1) cu_conv3(a, false);
+    else if (k3 && s.S == 2) cu_conv_s2(a, 3, 1);
+    else if (k2 && s.S == 2) cu_conv_s2(a, 2, 0);
+    else return false;
+  } else {
+    a.x0 = a.x1 = g.dy; a.C0 = a.C = s.Cout;
+    a.N = s.Cin; a.N0 = s.C0;
+    a.out1 = g.out1;
+    a.H = a.GH = s.Ho; a.W = a.GW = s.Wo; a.OH = s.H; a.OW = s.W;
+    if (k3 && s.S == 1) cu_conv3(a, true);
+    else if (s.S == 2 && s.H == 2 * s.Ho && s.W == 2 * s.Wo && (k3 || k2)) cu_adj_s2(a, s.KH, s.P);
+    else return false;
+  }
+  return cu_plan(a, s.KH * s.KW, smem);
+}
+
+// forward (DGRAD false) or data-gradient GEMM: k_conv_umma where the layer fits it (`packed`:
+// its weights); else the gathering kernels, tcgen05 when the net is configured for them
+template <bool DGRAD>
+int launch_gemm(const Net* u, const GemmArgs& a, const __nv_bfloat16* packed, cudaStream_t st) {
   const ConvShape& s = a.s;
+  ConvUmma c;
+  int smem = 0;
+  if (plan_umma<DGRAD>(a, packed, c, smem)) {
+    U_CK(launch_conv_umma(c, smem, u->umma_err, st));
+    return CDX_OK;
+  }
   const long long M = DGRAD ? (long long)s.N * s.H * s.W : (long long)s.N * s.Ho * s.Wo;
   const int NC = DGRAD ? s.Cin : s.Cout;
   const int K = DGRAD ? s.KH * s.KW * s.Cout : s.KH * s.KW * s.Cin;
@@ -906,13 +955,13 @@ int forward(Net* u, const float* inten, int count) {
       a.w = l.wt;
       a.out0 = l.pre;
       a.out1 = l.pre;
-      if ((e = launch_gemm<true>(u, a, u->st))) return e;
+      if ((e = launch_gemm<true>(u, a, l.pt, u->st))) return e;
     } else {
       a.x0 = act_of(u, l.in0);
       a.x1 = l.in1 >= 0 ? act_of(u, l.in1) : a.x0;
       a.w = l.wb;
       a.out0 = l.pre;
-      if ((e = launch_gemm<false>(u, a, u->st))) return e;
+      if ((e = launch_gemm<false>(u, a, l.pb, u->st))) return e;
     }
     const long long px = (long long)count * l.out_h * l.out_h;
     if (l.kind == L_HEAD) {
@@ -977,7 +1026,7 @@ int backward(Net* u, const float* amp_t, const float* ph_t, const float* sup_t, 
         f.out0 = u->L[l.in0].dact;
         f.acc0 = reached[l.in0];
         reached[l.in0] = 1;
-        if ((e = launch_gemm<false>(u, f, u->st))) return e;
+        if ((e = launch_gemm<false>(u, f, l.pb, u->st))) return e;
       }
     } else {
       a.x0 = act_of(u, l.in0);
@@ -997,7 +1046,7 @@ int backward(Net* u, const float* amp_t, const float* ph_t, const float* sup_t, 
           d.acc1 = reached[l.in1];
           reached[l.in1] = 1;
         }
-        if ((e = launch_gemm<true>(u, d, u->st))) return e;
+        if ((e = launch_gemm<true>(u, d, l.pt, u->st))) return e;
       }
     }
   }

@@ -42,9 +42,10 @@ typedef struct {
   float slope;        /* LeakyReLU negative slope */
   float support_weight; /* w_s */
   unsigned long long seed; /* weight initialisation */
-  int umma;           /* 1: forward and data-gradient convolutions on tcgen05/TMEM; 0 (default):
-                         warp-level mma.sync, faster for these channel counts (the weight gradient
-                         is mma.sync in both; the two give the same bits) */
+  int umma;           /* kernels of the forward and data-gradient convolutions whose channels do not fit the
+                         tcgen05 patch kernel (16 to 256, whole 16s; those always take it): 1 tcgen05 with
+                         gathered tiles, 0 (default) warp-level mma.sync.  The weight gradient is mma.sync.
+                         All of them give the same bits */
 } cdx_unet_config;
 
 int cdx_unet_config_default(cdx_unet_config* c);

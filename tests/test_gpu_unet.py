@@ -91,6 +91,32 @@ def test_group_norm_geometries_match_oracle(cdx, torch_cuda, n, levels, base, gr
     assert rel(g, g_ref) < 3e-2
 
 
+@pytest.mark.parametrize("n,levels,base,batch", [
+    (16, 2, 16, 1),      # grids smaller than a tile
+    (96, 3, 16, 1),      # 48 and 24 wide: half-filled last tiles
+    (48, 2, 32, 2),      # resident weights, three patch buffers
+    (32, 3, 64, 3),      # streamed weights, 256 channels in, four parity classes of 128
+])
+def test_convolution_tiles_match_oracle(cdx, torch_cuda, n, levels, base, batch):
+    """The tcgen05 patch convolutions at the edges of their tiles and plans, with the bounds of
+    test_gradients_match_fp64_oracle."""
+    torch = torch_cuda
+    from cdixx_gb300 import unet
+    I, amp, ph, sup = small_case(n, batch, seed=4)
+    p = U.init_params(n, levels, base, seed=5)
+    loss_ref, g_ref, out_ref = U.forward_backward(p, I, amp, ph, sup, n, levels, base, round_bf16=True)
+    with unet.UNet(n=n, levels=levels, base=base, batch=batch) as net:
+        net.set_params(p)
+        dev = [torch.from_numpy(x).cuda() for x in (I, amp, ph, sup)]
+        out = net.forward(dev[0]).cpu().numpy().transpose(0, 2, 3, 1)
+        loss = net.loss_backward(*dev)
+        g = net.grads().astype(np.float64)
+    rel = lambda a, b: np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-30)
+    assert rel(out, out_ref) < 5e-3
+    assert abs(loss - loss_ref) <= 2e-3 * abs(loss_ref)
+    assert rel(g, g_ref) < 3e-2
+
+
 def test_forward_model_matches_restatement(cdx, torch_cuda):
     from cdixx_gb300 import unet
     n, count, seed, first = 64, 3, 11, 5
