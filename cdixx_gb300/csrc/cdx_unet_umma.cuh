@@ -23,8 +23,8 @@
 // bounded; a role that gives up sets *err and the abort flag, which ends the others.
 //
 // Bound by HBM and the L2 (FP32 outputs, patches and streamed weights).  Batch 32 of
-// 256^2 (4 levels, 32 channels): the step's 26 launches take 3.4 ms (10.5 with the
-// gathering kernels), the network on 8 patterns 1.91 -> 1.21 ms as a whole.
+// 256^2 (4 levels, 32 channels): the step's 26 launches take 2.7 ms (10.5 with the
+// gathering kernels), the network on 8 patterns 1.91 -> 1.11 ms as a whole.
 #pragma once
 #include "cdx_umma.cuh"
 
@@ -33,8 +33,9 @@ namespace unet {
 
 constexpr int kCuTH = 16, kCuTW = 8;      // tile grid rows and columns of a CTA
 constexpr int kCuThreads = 320;
-constexpr int kCuSmem = 220 * 1024;       // dynamic shared memory a CTA may take
+constexpr int kCuSmem = 214 * 1024;       // dynamic shared memory a CTA may take
 constexpr int kCuStagesMax = 8, kCuPatchMax = 3;
+constexpr int kCuEpi = 20;                // floats a pixel's 16 channels take in the epilogue's staging (padded)
 
 struct ConvUmma {
   const __nv_bfloat16 *x0, *x1;           // input parts (channels [0, C0) and [C0, C))
@@ -75,6 +76,7 @@ __global__ void __launch_bounds__(kCuThreads, 3) k_conv_umma(const __grid_consta
       tfull[2], tempty[2], done;
   __shared__ unsigned tmem_base;
   __shared__ volatile int abort_flag;
+  __shared__ __align__(16) float epi[4 * 32 * kCuEpi];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int C8 = a.C >> 3, N = a.N;
   const unsigned plane = (unsigned)a.slots * 16, patch = plane * C8;
@@ -153,13 +155,16 @@ __global__ void __launch_bounds__(kCuThreads, 3) k_conv_umma(const __grid_consta
     }
   } else if (warp < 8) {
     // ------------------------------------------------------------ epilogue
-    const int ew = warp - 4, row = ew * 32 + lane;
+    // a warp's 32 grid pixels are four rows of eight; 16 channels at a time go through
+    // shared memory so that four lanes write the 64 bytes of a pixel (a lane writing its
+    // own pixel's 16-byte pieces left half sectors: 32 -> 32 at 256^2 x32, 161 -> 113 us)
+    const int ew = warp - 4;
+    float* tr = epi + ew * 32 * kCuEpi;
     int q = 0;
     bool failed = false;
     for (int t = blockIdx.x; t < tiles && !failed; t += gridDim.x) {
       const int img = t / (ty * tx), r = t - img * ty * tx;
-      const int gy = r / tx * kCuTH + (row >> 3), gx = (r % tx) * kCuTW + (row & 7);
-      const bool ok = gy < a.GH && gx < a.GW;
+      const int gy = r / tx * kCuTH + ew * 4, gx = (r % tx) * kCuTW + (lane >> 2);
       for (int cls = 0; cls < a.ncls; ++cls, ++q) {
         const int b = q & 1;
         if (!mbar_wait_or_abort(smem_u32(&tfull[b]), (unsigned)((q >> 1) & 1), &abort_flag)) {
@@ -179,20 +184,25 @@ __global__ void __launch_bounds__(kCuThreads, 3) k_conv_umma(const __grid_consta
               : "r"(ta)
               : "memory");
           asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-          if (ok) {
-            const bool second = c0 >= a.N0;
-            float4* o = reinterpret_cast<float4*>(second ? a.out1 + px * (N - a.N0) + (c0 - a.N0) : a.out0 + px * a.N0 + c0);
-            const bool add = second ? a.acc1 : a.acc0;
+          __syncwarp();   // the previous channels have been read
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              float4 f = make_float4(__uint_as_float(v[4 * k]), __uint_as_float(v[4 * k + 1]),
-                                     __uint_as_float(v[4 * k + 2]), __uint_as_float(v[4 * k + 3]));
-              if (add) {
-                const float4 e = o[k];
-                f = make_float4(e.x + f.x, e.y + f.y, e.z + f.z, e.w + f.w);
-              }
-              o[k] = f;
+          for (int k = 0; k < 4; ++k)
+            *reinterpret_cast<uint4*>(tr + lane * kCuEpi + 4 * k) = make_uint4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+          __syncwarp();
+          const bool second = c0 >= a.N0, add = second ? a.acc1 : a.acc0;
+          const int ch = second ? N - a.N0 : a.N0, c = (second ? c0 - a.N0 : c0) + 4 * (lane & 3);
+          float* out = (second ? a.out1 : a.out0) + px * ch + c;
+          const long long step = (long long)a.out_s * a.OW * ch;   // one grid row
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            if (gy + k >= a.GH || gx >= a.GW) continue;
+            float4 f = *reinterpret_cast<const float4*>(tr + (8 * k + (lane >> 2)) * kCuEpi + 4 * (lane & 3));
+            float4* o = reinterpret_cast<float4*>(out + k * step);
+            if (add) {
+              const float4 e = *o;
+              f = make_float4(e.x + f.x, e.y + f.y, e.z + f.z, e.w + f.w);
             }
+            *o = f;
           }
         }
         asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -315,11 +325,12 @@ inline bool cu_plan(ConvUmma& a, int taps, int& smem) {
   if (wall + 2 * patch <= kCuSmem * 3 / 4) {   // resident weights, and room for copies in flight
     a.nstage = 0;
     a.cch = a.C;
-    a.npatch = wall + 3 * patch <= kCuSmem / 2 ? 3 : 2;
+    a.npatch = wall + 3 * patch <= 100 * 1024 ? 3 : 2;   // two CTAs per SM either way where they fit
     smem = a.npatch * patch + wall;
     return true;
   }
-  a.cch = a.C < 32 ? 16 : 32;
+  a.cch = a.C;   // stages of about 16 KB: smaller ones spend the MMA lane on barriers
+  while (a.cch % 32 == 0 && a.cch * a.N * 2 > 16384) a.cch /= 2;
   const int stage = a.cch * a.N * 2;
   a.npatch = 2 * patch + 2 * stage <= kCuSmem ? 2 : 1;
   a.nstage = std::min(kCuStagesMax, (kCuSmem - a.npatch * patch) / stage);
@@ -341,7 +352,7 @@ inline cudaError_t launch_conv_umma(const ConvUmma& a, int smem, int* err, cudaS
   int cols = 32;
   while (cols < 2 * a.N) cols *= 2;
   // resident CTAs per SM: shared memory (228 KB, 1 KB reserved per CTA), TMEM columns, threads
-  const int per_sm = std::max(1, std::min({(228 * 1024) / (smem + 2048), 512 / cols, 3}));
+  const int per_sm = std::max(1, std::min({(228 * 1024) / (smem + 1024 + 11 * 1024), 512 / cols, 3}));
   const long long tiles = (long long)a.nimg * ((a.GH + kCuTH - 1) / kCuTH) * ((a.GW + kCuTW - 1) / kCuTW);
   const int grid = (int)std::min<long long>(tiles, (long long)per_sm * sm_count());
   k_conv_umma<<<grid, kCuThreads, smem, st>>>(a, err);
