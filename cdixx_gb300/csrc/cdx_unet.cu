@@ -916,7 +916,15 @@ int launch_wgrad(Net* u, GemmArgs a, const Layer& l) {
   if ((size_t)(splits * s.Cout * K) > u->wpart_cap) return set_error(CDX_ERR_STATE, "wgrad scratch too small");
   a.out0 = u->wpart;
   a.m_per_split = (int)mps;
-  k_conv_wgrad<<<dim3(tx, ty, (unsigned)splits), 128, 0, u->st>>>(a);
+  WgradUmma w{};
+  w.x0 = a.x0; w.x1 = a.x1; w.dy = a.dy; w.part = u->wpart;
+  w.C0 = s.C0; w.Cin = s.Cin; w.Cout = s.Cout;
+  w.H = s.H; w.W = s.W; w.Ho = s.Ho; w.Wo = s.Wo;
+  w.KH = s.KH; w.KW = s.KW; w.S = s.S; w.P = s.P;
+  w.M = (int)M;
+  w.m_per_split = (int)mps;
+  if (wg_plan(w, (int)splits, sm_count())) U_CK(launch_wgrad_umma(w, (int)splits, u->umma_err, u->st));
+  else k_conv_wgrad<<<dim3(tx, ty, (unsigned)splits), 128, 0, u->st>>>(a);
   const long long tot = (long long)l.wco_r * l.k * l.k * l.wci_r;
   k_wgrad_reduce<<<grid_for(tot), kThreads, 0, u->st>>>(u->wpart, (int)splits, l.wco_r, l.wci_r, l.wco_p, l.wci_p,
                                                          l.k * l.k, u->grads + l.w_off);

@@ -420,5 +420,231 @@ inline void cu_adj_s2(ConvUmma& a, int k, int p) {
   }
 }
 
+// ------------------------------------------------------------------- wgrad
+// dW[co][tap][ci] = sum over output pixels m of dY[m][co] X[m at tap][ci].  Both
+// operands are the channel planes above with the pixels as K (MN-major: a core matrix
+// is eight pixels of eight channels), so one row segment of X serves the KW taps of a
+// filter row at shifted starts.  A CTA takes one filter row, up to 128 channels of one
+// side as M and up to 128 of the other as N (KW accumulators of N columns), and one
+// split of the pixels, which it walks in order in steps of 16, as k_conv_wgrad does:
+// the partial sums are the same, bit for bit.  Rows of M and columns of N past the
+// channels multiply whatever lies behind the planes and are not read back.
+// Bound by the operands' reads from shared memory (an MMA of M = 128 takes 32 cycles
+// whatever N up to 64).  Batch 32 of 256^2: the step's 15 launches 8.5 -> 3.9 ms.
+constexpr int kWgStages = 4, kWgAhead = 2;
+constexpr int kWgThreads = 160;     // warps 0-3 copy and then drain the accumulators, warp 4 issues the MMAs
+
+struct WgradUmma {
+  const __nv_bfloat16 *x0, *x1, *dy;   // X parts (channels [0, C0) and [C0, Cin)), dY
+  float* part;                         // [splits][Cout][KH * KW * Cin]
+  int C0, Cin, Cout, H, W, Ho, Wo, KH, KW, S, P;
+  int M, m_per_split;                  // output pixels, per split
+  int m_is_x;                          // M side: X's channels (else dY's)
+  int mt, nt, nn;                      // M tiles, N tiles, channels of an N tile
+  int xslots, yslots, xpl, ypl;        // slots of a plane and planes of a stage, X and dY
+  int seg;                             // output pixels of a stage (of one row)
+  int stage, smem;                     // bytes of a stage, of the launch
+};
+
+// MN-major no-swizzle operand: SBO from eight channels to the next, LBO from eight pixels to the next
+__device__ __forceinline__ uint64_t wg_desc(unsigned saddr, unsigned plane) {
+  return (uint64_t)((saddr >> 4) & 0x3FFF) | (uint64_t)(128 >> 4) << 16 | (uint64_t)(plane >> 4) << 32 |
+         (uint64_t)1 << 46;
+}
+
+__global__ void __launch_bounds__(kWgThreads, 1) k_wgrad_umma(const __grid_constant__ WgradUmma a, int* __restrict__ err) {
+  using namespace umma;
+  extern __shared__ __align__(128) unsigned char sm[];
+  __shared__ __align__(8) uint64_t full[kWgStages], empty[kWgStages], done;
+  __shared__ unsigned tmem_base;
+  __shared__ volatile int abort_flag;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int ky = blockIdx.x % a.KH, mtile = blockIdx.x / a.KH % a.mt, ntile = blockIdx.x / a.KH / a.mt;
+  const int mb = blockIdx.y * a.m_per_split, me = min(a.M, mb + a.m_per_split);
+  const int cx0 = (a.m_is_x ? mtile * 128 : ntile * a.nn), cy0 = (a.m_is_x ? ntile * a.nn : mtile * 128);
+  const int nx = min(a.m_is_x ? 128 : a.nn, a.Cin - cx0), ny = min(a.m_is_x ? a.nn : 128, a.Cout - cy0);
+  const unsigned xplane = (unsigned)a.xslots * 16, yplane = (unsigned)a.yslots * 16;
+  const int ncol = (a.nn + 15) & ~15;                       // columns of an accumulator
+  int cols = 32;
+  while (cols < a.KW * ncol) cols *= 2;
+
+  if (warp == 4) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_base)),
+                 "r"(cols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+  }
+  if (tid == 0) {
+    for (int i = 0; i < kWgStages; ++i) { mbar_init(smem_u32(&full[i]), 128); mbar_init(smem_u32(&empty[i]), 1); }
+    mbar_init(smem_u32(&done), 1);
+    abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  const unsigned tmem = tmem_base, base = smem_u32(sm);
+  auto give_up = [&]() {
+    abort_flag = 1;
+    atomicExch(err, 1);
+  };
+  const int hw = a.Ho * a.Wo, par = a.seg + (a.KW > 1);    // slots of one column parity (stride 2)
+
+  if (warp < 4) {
+    // ------------------------------------------------------------ copies
+    const int xp = nx / 8, yp = ny / 8, xper = 128 / xp, yper = 128 / yp;
+    const int xc = tid % xp, xi = tid / xp, yc = tid % yp, yi = tid / yp;
+    const int c = cx0 + xc * 8, ch = c < a.C0 ? a.C0 : a.Cin - a.C0;
+    const __nv_bfloat16* xsrc = c < a.C0 ? a.x0 + c : a.x1 + (c - a.C0);
+    const __nv_bfloat16* ysrc = a.dy + cy0 + yc * 8;
+    int g = 0;
+    bool failed = false;
+    for (int m = mb; m < me && !failed; ++g) {
+      const int s = g % kWgStages, use = g / kWgStages;
+      if (use > 0 && !mbar_wait_or_abort(smem_u32(&empty[s]), (unsigned)((use - 1) & 1), &abort_flag)) {
+        failed = true;
+        break;
+      }
+      const int img = m / hw, r = m - img * hw, oy = r / a.Wo, ox = r - oy * a.Wo;
+      const int len = min(min(a.seg, a.Wo - ox), me - m);
+      const unsigned xd = base + s * a.stage + xc * xplane, yd = base + s * a.stage + a.xpl * xplane + yc * yplane;
+      const int y = oy * a.S - a.P + ky, x0 = ox * a.S - a.P, npx = (len - 1) * a.S + a.KW;
+      const bool row = y >= 0 && y < a.H;
+      const __nv_bfloat16* xrow = xsrc + ((long long)img * a.H + (row ? y : 0)) * a.W * ch;
+      if (xi < xper)
+        for (int p = xi; p < npx; p += xper) {
+          const int x = x0 + p, slot = a.S == 1 ? p : (p & 1) * par + (p >> 1);
+          const bool ok = row && x >= 0 && x < a.W;
+          umma::cp16(xd + slot * 16, ok ? (const void*)(xrow + (long long)x * ch) : (const void*)a.dy, ok);
+        }
+      if (yi < yper)
+        for (int p = yi; p < len; p += yper) umma::cp16(yd + p * 16, ysrc + (long long)(m + p) * a.Cout, true);
+      umma::cp_commit();
+      if (g >= kWgAhead) {
+        umma::cp_wait<kWgAhead>();
+        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+        mbar_arrive(smem_u32(&full[(g - kWgAhead) % kWgStages]));
+      }
+      m += len;
+    }
+    umma::cp_wait<0>();
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    if (failed) {
+      if (lane == 0) give_up();
+    } else {
+      for (int q = g > kWgAhead ? g - kWgAhead : 0; q < g; ++q) mbar_arrive(smem_u32(&full[q % kWgStages]));
+    }
+    // ------------------------------------------------------------ partial sums
+    if (!mbar_wait_or_abort(smem_u32(&done), 0, &abort_flag) || abort_flag) {
+      if (lane == 0) give_up();
+    } else {
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      const int K = a.KH * a.KW * a.Cin, row = warp * 32 + lane, nm = a.m_is_x ? nx : ny, nv = a.m_is_x ? ny : nx;
+      float* part = a.part + (long long)blockIdx.y * a.Cout * K;
+      for (int t = 0; t < a.KW; ++t)
+        for (int c0 = 0; c0 < ncol; c0 += 16) {
+          uint32_t v[16];
+          const unsigned ta = tmem + ((unsigned)(warp * 32) << 16) + (unsigned)(t * ncol + c0);
+          asm volatile(
+              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+              : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+              : "r"(ta)
+              : "memory");
+          asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+          if (row >= nm) continue;
+          const int k = (ky * a.KW + t) * a.Cin + cx0;
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (c0 + j < nv) {
+              const float f = mb < me ? __uint_as_float(v[j]) : 0.f;
+              if (a.m_is_x) part[(long long)(cy0 + c0 + j) * K + k + row] = f;
+              else part[(long long)(cy0 + row) * K + k + c0 + j] = f;
+            }
+        }
+    }
+  } else {
+    // ------------------------------------------------------------ MMA lane
+    if (lane == 0) {
+      // A and B MN-major (bits 15, 16)
+      const uint32_t idesc = idesc_bf16(128, ncol) | (1u << 15) | (1u << 16);
+      int g = 0;
+      bool failed = false;
+      for (int m = mb; m < me; ++g) {
+        const int s = g % kWgStages, ox = m % a.Wo, len = min(min(a.seg, a.Wo - ox), me - m);
+        if (!mbar_wait_or_abort(smem_u32(&full[s]), (unsigned)((g / kWgStages) & 1), &abort_flag)) {
+          failed = true;
+          break;
+        }
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        const unsigned xa = base + s * a.stage, ya = xa + a.xpl * xplane;
+        for (int p = 0; p < len; p += 16)
+          for (int t = 0; t < a.KW; ++t) {
+            const int slot = a.S == 1 ? p + t : (t & 1) * par + p + (t >> 1);
+            const uint64_t dx = wg_desc(xa + slot * 16, xplane), dy = wg_desc(ya + p * 16, yplane);
+            mma_f16(tmem + t * ncol, a.m_is_x ? dx : dy, a.m_is_x ? dy : dx, idesc, g > 0 || p > 0);
+          }
+        mma_commit(smem_u32(&empty[s]));
+        m += len;
+      }
+      if (failed) give_up();
+      mma_commit(smem_u32(&done));
+    }
+    __syncwarp();
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  if (warp == 4) {
+    if (!mbar_wait(smem_u32(&done), 0) && lane == 0) atomicExch(err, 1);
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(cols) : "memory");
+  }
+}
+
+// Tiles and shared memory of a launch over `splits` splits; false: the layer does not fit
+// (16 output pixels of a K step have to lie in one row, whole 8-channel planes).
+inline bool wg_plan(WgradUmma& a, int splits, int sms) {
+  if (a.Wo % 16 || a.Cin % 8 || a.Cout % 8 || a.C0 % 8 || a.KW > 3 || a.S > 2 || a.m_per_split % 16) return false;
+  a.m_is_x = a.Cin >= a.Cout;   // the larger side fills M
+  const int mc = a.m_is_x ? a.Cin : a.Cout, nc = a.m_is_x ? a.Cout : a.Cin;
+  a.mt = (mc + 127) / 128;
+  auto sized = [&](int nn, int seg) {
+    a.nn = std::min(nc, nn);
+    a.nt = (nc + a.nn - 1) / a.nn;
+    a.seg = seg;
+    a.xpl = std::min(a.m_is_x ? 128 : a.nn, a.Cin) / 8;
+    a.ypl = std::min(a.m_is_x ? a.nn : 128, a.Cout) / 8;
+    a.xslots = (a.S == 1 ? seg + a.KW - 1 : 2 * (seg + (a.KW > 1))) | 1;
+    a.yslots = seg | 1;
+    a.stage = (a.xpl * a.xslots + a.ypl * a.yslots) * 16;
+    // behind the last stage: what the unused rows and columns read (16 planes of either side at most)
+    a.smem = kWgStages * a.stage + 16 * std::max(a.xslots, a.yslots) * 16;
+    return a.KH * a.mt * a.nt * splits <= sms ? kCuSmem : kCuSmem / 2 - 8 * 1024;   // one CTA per SM, or two
+  };
+  // 128 columns of N unless that leaves SMs without a CTA; the longest segments that fit
+  for (int nn = nc > 64 && a.KH * a.mt * ((nc + 127) / 128) * splits < sms ? 64 : 128; nn >= 64; nn -= 64)
+    for (int seg = 256; seg >= 64; seg /= 2)
+      if (a.Wo % seg == 0 || seg == 64) {
+        const int budget = sized(nn, seg);
+        if (a.smem <= (seg == 64 ? kCuSmem : budget)) return true;
+      }
+  return false;
+}
+
+inline cudaError_t launch_wgrad_umma(const WgradUmma& a, int splits, int* err, cudaStream_t st) {
+  static std::atomic<unsigned long long> done{0};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+  if (!(done.load(std::memory_order_acquire) & bit)) {
+    if ((e = cudaFuncSetAttribute(k_wgrad_umma, cudaFuncAttributeMaxDynamicSharedMemorySize, kCuSmem)) != cudaSuccess)
+      return e;
+    done.fetch_or(bit, std::memory_order_release);
+  }
+  k_wgrad_umma<<<dim3(a.KH * a.mt * a.nt, splits), kWgThreads, a.smem, st>>>(a, err);
+  return cudaGetLastError();
+}
+
 }  // namespace unet
 }  // namespace cdx

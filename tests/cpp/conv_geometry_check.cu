@@ -73,7 +73,52 @@ static void check(const char* form, const ConvUmma& a, int k, int s, int p, bool
     }
 }
 
+// weight gradient: the slots of one stage (a row segment), and the shared-memory plan
+static void check_wgrad(int KW, int S, int P) {
+  WgradUmma a{};
+  a.KH = a.KW = KW; a.S = S; a.P = P;
+  a.m_per_split = 32;
+  for (int Wo : {16, 64, 256})
+  for (int splits : {1, 64})
+  for (int Cin = 8; Cin <= 520; Cin += 8)
+    for (int Cout = 8; Cout <= 520; Cout += 8) {
+      a.Cin = a.C0 = Cin; a.Cout = Cout; a.Wo = Wo;
+      if (!wg_plan(a, splits, 152)) { fail("wgrad", "a layer of whole 8s does not fit"); continue; }
+      const int mc = a.m_is_x ? Cin : Cout, nc = a.m_is_x ? Cout : Cin, ncol = (a.nn + 15) & ~15;
+      if (a.mt * 128 < mc || a.nt * a.nn < nc || KW * ncol > 512 || ncol > 256) fail("wgrad", "tiles");
+      if (a.smem > kCuSmem || a.seg % 16) fail("wgrad", "shared-memory plan");
+      // operands read 16 (M) and ncol / 8 (N) planes from the start of the last stage's halves
+      const long long last = (long long)(kWgStages - 1) * a.stage;
+      const int xr = a.m_is_x ? 16 : ncol / 8, yr = a.m_is_x ? ncol / 8 : 16;
+      if (last + 16LL * xr * a.xslots > a.smem || last + 16LL * a.xpl * a.xslots + 16LL * yr * a.yslots > a.smem)
+        fail("wgrad", "an operand ends past the shared memory");
+      if (a.xpl * 8 < std::min(a.m_is_x ? 128 : a.nn, Cin) || a.ypl * 8 < std::min(a.m_is_x ? a.nn : 128, Cout))
+        fail("wgrad", "planes");
+    }
+  for (int C = 8; C <= 128; C *= 4) {
+  a.Cin = a.C0 = a.Cout = C; a.Wo = 256;
+  if (!wg_plan(a, 64, 152)) fail("wgrad", "plan");
+  const int par = a.seg + (KW > 1);
+  for (int len = 16; len <= a.seg; len += 16) {
+    std::map<int, int> filled;
+    for (int p = 0; p < (len - 1) * S + KW; ++p) {
+      const int slot = S == 1 ? p : (p & 1) * par + (p >> 1);
+      if (slot >= a.xslots || filled.count(slot)) fail("wgrad", "slot");
+      filled[slot] = p;
+    }
+    for (int p = 0; p < len; p += 16)
+      for (int t = 0; t < KW; ++t)
+        for (int i = 0; i < 16; ++i) {
+          const int slot = (S == 1 ? p + t : (t & 1) * par + p + (t >> 1)) + i;
+          if (!filled.count(slot) || filled[slot] != (p + i) * S + t) fail("wgrad", "tap pixel");
+        }
+    if (len > a.yslots) fail("wgrad", "dY slots");
+  }
+  }
+}
+
 int main() {
+  check_wgrad(3, 1, 1); check_wgrad(3, 2, 1); check_wgrad(2, 2, 0); check_wgrad(1, 1, 0);
   ConvUmma a{};
   cu_conv3(a, false); check("3x3", a, 3, 1, 1, false);
   cu_conv3(a, true); check("3x3 data gradient", a, 3, 1, 1, true);
