@@ -107,9 +107,13 @@ __device__ __forceinline__ long long pty_tiled(int r, int c, int rows, int tl) {
 }
 
 // Row kernels stage the CTA's object-window rows and probe rows in shared
-// memory with 8-byte cp.async (the window may start at any column; pixels
-// outside the object are zero-filled), line stride N + 8 so the lines a warp
-// reads together fall on different bank halves.
+// memory with cp.async (pixels outside the object are zero-filled), line stride
+// N + 8 so the lines a warp reads together fall on different bank halves.  What
+// the launch before does not write is loaded ahead of the wait for it: the scan
+// index and window always (the sweep counter and the windows change between
+// sweeps), the probe from the second position of a sweep on, the pattern, and in
+// the update pass the window too (the column pass is in between).  A position
+// chain of three kernels is latency (512^2 probe, 8 positions: 0.186 -> 0.171 ms per sweep).
 template <int N>
 struct PtyRow {
   static constexpr int SN = N + 8;
@@ -119,22 +123,37 @@ struct PtyRow {
   static constexpr int SMEM = RGeom<FGeom<N>>::SMEM_ROW_LINES + STAGE;
 };
 
+// The CTA's probe rows (16-byte pieces; the rows of an N-wide frame are aligned).
 template <int N>
-__device__ __forceinline__ void pty_stage_rows(const PtyArgs& a, float2* o_s, float2* p_s, int row0, int nrows,
-                                               int2 w) {
+__device__ __forceinline__ void pty_stage_probe(const PtyArgs& a, float2* p_s, int row0, int nrows) {
+  using G = FGeom<N>;
+  constexpr int L = G::L, T = G::T, SN = PtyRow<N>::SN;
+  for (int e = threadIdx.x; e < L * N / 2; e += T) {
+    const int l = 2 * e / N, c = 2 * e - l * N;
+    const bool ok = l < nrows;
+    cp_async16(p_s + l * SN + c, ok ? (const void*)(a.probe + (long long)(row0 + l) * N + c) : (const void*)a.probe, ok);
+  }
+}
+// The CTA's rows of the object window, zero outside the object: 16-byte pieces where the
+// window starts on an even column of an even-width object and ends inside it, else 8-byte ones.
+template <int N>
+__device__ __forceinline__ void pty_stage_window(const PtyArgs& a, float2* o_s, int row0, int nrows, int2 w) {
   using G = FGeom<N>;
   constexpr int L = G::L, T = G::T, SN = PtyRow<N>::SN;
   const long long OC = a.obj_cols;
-  for (int e = threadIdx.x; e < L * N; e += T) {
-    const int l = e / N, c = e - l * N;
-    const int row = row0 + l;
-    const bool rok = l < nrows;
-    const int ox = w.x + row, oy = w.y + c;
-    const bool inb = rok && ox >= 0 && ox < a.obj_rows && oy >= 0 && oy < a.obj_cols;
-    cp_async8(o_s + l * SN + c, inb ? (const void*)(a.obj + ox * OC + oy) : (const void*)a.obj, inb);
-    cp_async8(p_s + l * SN + c, rok ? (const void*)(a.probe + (long long)row * N + c) : (const void*)a.probe, rok);
+  if (((w.y | a.obj_cols) & 1) == 0 && w.y >= 0 && w.y + N <= a.obj_cols) {
+    for (int e = threadIdx.x; e < L * N / 2; e += T) {
+      const int l = 2 * e / N, c = 2 * e - l * N, ox = w.x + row0 + l;
+      const bool ok = l < nrows && ox >= 0 && ox < a.obj_rows;
+      cp_async16(o_s + l * SN + c, ok ? (const void*)(a.obj + ox * OC + w.y + c) : (const void*)a.obj, ok);
+    }
+    return;
   }
-  cp_commit();
+  for (int e = threadIdx.x; e < L * N; e += T) {
+    const int l = e / N, c = e - l * N, ox = w.x + row0 + l, oy = w.y + c;
+    const bool ok = l < nrows && ox >= 0 && ox < a.obj_rows && oy >= 0 && oy < a.obj_cols;
+    cp_async8(o_s + l * SN + c, ok ? (const void*)(a.obj + ox * OC + oy) : (const void*)a.obj, ok);
+  }
 }
 
 // ------------------------------------------------------- forward row pass
@@ -147,14 +166,17 @@ __global__ void __launch_bounds__(FGeom<N>::T, PtyRow<N>::MINB) pty_fwd_rk(PtyAr
   using FL = RLast<G, 0>;
   constexpr int SN = PtyRow<N>::SN, LD = PtyRow<N>::LD;
   extern __shared__ float2 smem[];
-  pdl_wait_and_release();
   float2* o_s = smem + L * LD;
   float2* p_s = o_s + L * SN;
   const int row0 = blockIdx.x * L;
   const int nrows = min(L, a.rows - row0);
   const int cb = row_cb_pick(a.tl, rfft_cb_max<N>());
-  const int si = a.order[*a.iter * a.nscan + a.k];
-  pty_stage_rows<N>(a, o_s, p_s, row0, nrows, a.win[si]);
+  const int2 w = a.win[a.order[*a.iter * a.nscan + a.k]];
+  if (a.k > 0) pty_stage_probe<N>(a, p_s, row0, nrows);
+  pdl_wait_and_release();
+  if (a.k == 0) pty_stage_probe<N>(a, p_s, row0, nrows);   // the first position follows the probe's own kernels
+  pty_stage_window<N>(a, o_s, row0, nrows, w);
+  cp_commit();
   cp_wait<0>();
   __syncthreads();
   float2 v0[F0::B][F0::R];
@@ -189,7 +211,6 @@ __global__ void __launch_bounds__(FGeom<N>::T, RGeom<FGeom<N>>::MINB_COL) pty_co
   using FL = RLast<G, 0>;
   using IL = RLast<G, 1>;
   extern __shared__ float2 smem[];
-  pdl_wait_and_release();
   const int c0 = blockIdx.x * L;
   const int ncols = min(L, a.cols - c0);
   const long long tile = (long long)blockIdx.x * N * L;
@@ -217,6 +238,7 @@ __global__ void __launch_bounds__(FGeom<N>::T, RGeom<FGeom<N>>::MINB_COL) pty_co
     }
     cp_commit();
   }
+  pdl_wait_and_release();
   float2 v0[F0::B][F0::R];
 #pragma unroll
   for (int b = 0; b < F0::B; ++b) {
@@ -264,16 +286,17 @@ __global__ void __launch_bounds__(FGeom<N>::T, PtyRow<N>::MINB) pty_upd_rk(PtyAr
   using FL = RLast<G, 0>;
   constexpr int SN = PtyRow<N>::SN, LD = PtyRow<N>::LD;
   extern __shared__ float2 smem[];
-  pdl_wait_and_release();
   float2* o_s = smem + L * LD;
   float2* p_s = o_s + L * SN;
   const int row0 = blockIdx.x * L;
   const int nrows = min(L, a.rows - row0);
   const int cb = row_cb_pick(a.tl, rfft_cb_max<N>());
-  const int si = a.order[*a.iter * a.nscan + a.k];
-  const int2 w = a.win[si];
+  const int2 w = a.win[a.order[*a.iter * a.nscan + a.k]];
   const long long OC = a.obj_cols;
-  pty_stage_rows<N>(a, o_s, p_s, row0, nrows, w);   // lands during the inverse FFT
+  pty_stage_probe<N>(a, p_s, row0, nrows);   // land during the inverse FFT
+  pty_stage_window<N>(a, o_s, row0, nrows, w);
+  cp_commit();
+  pdl_wait_and_release();
   float2 v0[F0::B][F0::R];
 #pragma unroll
   for (int b = 0; b < F0::B; ++b) {

@@ -300,7 +300,6 @@ __global__ void __launch_bounds__(G::T, RGeom<G>::MINB_COL) col_pass_rk(ColArgs 
   static_assert(FL::R == RFirst<G, 1>::R && FL::B == RFirst<G, 1>::B, "plan 1 starts where plan 0 ends");
   extern __shared__ float2 smem[];
   __shared__ double red[T / 32];
-  pdl_wait_and_release();
   const float2* __restrict__ tw = a.tw;
   float2* buf = smem;
   const int c0 = blockIdx.x * L;
@@ -308,20 +307,14 @@ __global__ void __launch_bounds__(G::T, RGeom<G>::MINB_COL) col_pass_rk(ColArgs 
   const long long C = a.cols;
   const long long tile = (long long)blockIdx.x * N * L;
 
-  if (a.state) {
-    const int f = a.state[blockIdx.y].flags;
-    if (f & 6) {
-      if ((f & 4) == 0 && threadIdx.x == 0) atomicOr(&a.state[blockIdx.y].flags, 4);
-      return;
-    }
-  }
   constexpr bool iter = MODE == COL_ITER;
   float* amp_s = reinterpret_cast<float*>(smem + L * G::LD);
   float* int_s = amp_s + L * N;
   float* bs_s = int_s + L * N;
   const long long aux = (long long)blockIdx.y * a.aux_stride + tile;
   // the tile's sqrt(I) (and I, beamstop for PROJ_CCD): contiguous runs of L*N
-  // floats, one bulk copy each, landing during the forward transform
+  // floats, one bulk copy each, started before the wait for the row pass (which
+  // does not write them) and landing during the forward transform
   __shared__ uint64_t stage_bar;
   if constexpr (iter) {
     if constexpr (bulk_staging<N>()) {
@@ -345,6 +338,18 @@ __global__ void __launch_bounds__(G::T, RGeom<G>::MINB_COL) col_pass_rk(ColArgs 
         }
       }
       cp_commit();
+    }
+  }
+  pdl_wait_and_release();
+  if (a.state) {
+    const int f = a.state[blockIdx.y].flags;
+    if (f & 6) {
+      if ((f & 4) == 0 && threadIdx.x == 0) atomicOr(&a.state[blockIdx.y].flags, 4);
+      if constexpr (iter) {   // the copies land before the CTA ends
+        if constexpr (bulk_staging<N>()) bulk_wait(&stage_bar, a.err);
+        else cp_wait<0>();
+      }
+      return;
     }
   }
   const float2* in = a.in + (long long)blockIdx.y * a.in_stride;
@@ -569,6 +574,15 @@ __device__ __forceinline__ void row_pass_body(const RowArgs& a) {
     }
     cp_commit();
   }
+  // support words and rho were last written before the column pass: only W has to be waited for
+  pdl_wait_and_release();
+  if (a.state && (a.state[blockIdx.y].flags & 4)) {   // frozen pattern: the copies land, nothing is computed
+    if constexpr (iter) {
+      cp_wait<0>();
+      if constexpr (bulk_rho && !rho_in_buf) bulk_wait(&rho_bar, a.err);
+    }
+    return;
+  }
   const float2* in = a.in + (long long)blockIdx.y * a.in_stride;
   const long long R = a.rows;
   auto goff = [&](bool t, int l, int c) -> long long {
@@ -682,8 +696,6 @@ __device__ __forceinline__ void row_pass_body(const RowArgs& a) {
 // holds a single update and no switch.
 template <class G, int MODE, int ALGO, bool SQ = false>
 __global__ void __launch_bounds__(G::T, MODE == ROW_FFT ? RGeom<G>::MINB_ROW_FFT : RGeom<G>::MINB_ROW) row_pass_rk(RowArgs a) {
-  pdl_wait_and_release();
-  if (a.state && (a.state[blockIdx.y].flags & 4)) return;   // frozen pattern
   row_pass_body<G, MODE, ALGO, SQ>(a);
 }
 // the compile-time layout of row_pass_rk<..., true> applies to these arguments
