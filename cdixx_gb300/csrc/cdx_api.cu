@@ -153,10 +153,9 @@ void rect_of(cdx_ctx* c) {
 
 int reset_support(cdx_ctx* c, int idx, int count) {
   const long long off = (long long)idx * c->npx;
-  CDX_CK(rect_support(c->spt + off, c->rows, c->cols, count, c->sx, c->sy, c->ex, c->ey, c->st));
-  // bits with the current threshold of each pattern
-  CDX_CK(support_bits(c->spt + off, c->dstate + idx, 0.f, c->mask + (long long)idx * c->rows * c->wpr, c->rows,
-                      c->cols, count, c->st));
+  // with the current threshold of each pattern
+  CDX_CK(rect_support(c->spt + off, c->dstate + idx, c->mask + (long long)idx * c->rows * c->wpr, c->rows, c->cols,
+                      count, c->sx, c->sy, c->ex, c->ey, c->st));
   return CDX_OK;
 }
 
@@ -1123,8 +1122,7 @@ int cdx_set_pattern(cdx_ctx* c, int idx, const float* inten, int where, int layo
   if (e) return e;
   if (layout == CDX_CENTERED) CDX_CK(convert_fo_real(c->inten + off, c->inten + off, c->rows, c->cols, 1, c->st));
   if (scale != 1.f) CDX_CK(scale_real(c->inten + off, scale, c->npx, c->st));
-  CDX_CK(to_tiled(c->inten + off, c->inten_t + toff, c->rows, c->cols, c->tl, c->wstride, 1, c->st));
-  CDX_CK(amp_from_pattern(c->inten_t + toff, c->amp_t + toff, c->wstride, c->st));
+  CDX_CK(to_tiled(c->inten + off, c->inten_t + toff, c->amp_t + toff, c->rows, c->cols, c->tl, c->st));
   CDX_CK(pattern_amp_sum(c->amp_t + toff, c->wstride, 1, c->part, kRedBlocks, c->dstate + idx, c->st));
   CDX_CK(cudaStreamSynchronize(c->st));
   c->have_pattern[idx] = 1;
@@ -1144,7 +1142,7 @@ int cdx_set_beamstop(cdx_ctx* c, int idx, const float* bs, int where, int layout
   int e = copy_in(c->bs + off, bs, sizeof(float) * c->npx, where, c->st);
   if (e) return e;
   if (layout == CDX_CENTERED) CDX_CK(convert_fo_real(c->bs + off, c->bs + off, c->rows, c->cols, 1, c->st));
-  CDX_CK(to_tiled(c->bs + off, c->bs_t + toff, c->rows, c->cols, c->tl, c->wstride, 1, c->st));
+  CDX_CK(to_tiled(c->bs + off, c->bs_t + toff, nullptr, c->rows, c->cols, c->tl, c->st));
   c->gkey.clear();
   CDX_CK(cudaStreamSynchronize(c->st));
   return CDX_OK;

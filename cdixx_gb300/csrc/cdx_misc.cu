@@ -74,26 +74,37 @@ cudaError_t convert_fo_complex(const float2* in, float2* out, int rows, int cols
 }
 
 // Row-major (rows x cols) -> column-tiled with tile width 2^tl (padding columns
-// of the last tile set to 0).  `out_stride` elements between patterns.
-__global__ void k_to_tiled(const float* __restrict__ in, float* __restrict__ out, int rows, int cols, int tl,
-                           long long out_stride, int batch) {
-  const int tw = 1 << tl;
-  const int cp = ((cols + tw - 1) >> tl) << tl;
-  const long long per = (long long)rows * cp;
-  for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < per * batch;
-       g += (long long)gridDim.x * blockDim.x) {
-    const long long p = g / per, i = g - p * per;
-    // i enumerates the tiled array: tile, row, lane
-    const long long tile = i / ((long long)rows << tl);
-    const long long rem = i - tile * ((long long)rows << tl);
-    const int r = (int)(rem >> tl), c = (int)(tile << tl) + (int)(rem & (tw - 1));
-    out[p * out_stride + i] = c < cols ? in[p * (long long)rows * cols + (long long)r * cols + c] : 0.f;
+// of the last tile set to 0), and sqrt(I) of the result (as k_amp; may be null).
+// 32 x 32 blocks go through shared memory so that rows are read in whole lines
+// (tile-order reads of 2-column tiles took 19 us for 2048^2 and the square root
+// 8 more; now 11.2 in all).
+__global__ void __launch_bounds__(256) k_to_tiled(const float* __restrict__ in, float* __restrict__ out,
+                                                  float* __restrict__ amp, int rows, int cols, int cp, int tl) {
+  __shared__ float t[32][33];
+  const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int r = r0 + ty + 8 * k, c = c0 + tx;
+    t[ty + 8 * k][tx] = r < rows && c < cols ? in[(long long)r * cols + c] : 0.f;
+  }
+  __syncthreads();
+  // element e of the block in tiled order: tile of the block, row, lane of the tile (tiles wider
+  // than the block: its 32 columns of one)
+  const int wl = min(tl, 5);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int e = threadIdx.x + 256 * k, lane = e & ((1 << wl) - 1), rr = (e >> wl) & 31, cc = ((e >> (wl + 5)) << wl) + lane;
+    const int r = r0 + rr, c = c0 + cc;
+    if (r >= rows || c >= cp) continue;
+    const float v = t[rr][cc];
+    const long long o = (((long long)(c >> tl) * rows + r) << tl) + (c & ((1 << tl) - 1));
+    out[o] = v;
+    if (amp) amp[o] = v > 0.f ? sqrtf(v) : 0.f;
   }
 }
-cudaError_t to_tiled(const float* in, float* out, int rows, int cols, int tl, long long out_stride, int batch,
-                     cudaStream_t st) {
+cudaError_t to_tiled(const float* in, float* out, float* amp, int rows, int cols, int tl, cudaStream_t st) {
   const int cp = ((cols + (1 << tl) - 1) >> tl) << tl;
-  k_to_tiled<<<grid1d((long long)rows * cp * batch, 256), 256, 0, st>>>(in, out, rows, cols, tl, out_stride, batch);
+  k_to_tiled<<<dim3((cp + 31) / 32, (rows + 31) / 32), 256, 0, st>>>(in, out, amp, rows, cols, cp, tl);
   return cudaGetLastError();
 }
 
@@ -130,43 +141,68 @@ cudaError_t apply_support(float2* rho, const float2* rhop, const float* spt, flo
 }
 
 // ------------------------------------------------------------------ supports
-// createMask<rect> (src/gpu/cudaConfig.cu:1291-1300): 1 inside [sx,ex) x [sy,ey).
-__global__ void k_rect(float* __restrict__ spt, int rows, int cols, int batch, int sx, int sy, int ex, int ey) {
-  const long long npx = (long long)rows * cols;
-  for (long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x; g < npx * batch; g += (long long)gridDim.x * blockDim.x) {
-    const long long i = g % npx;
-    const int x = (int)(i / cols), y = (int)(i - (long long)x * cols);
-    spt[g] = (x >= sx && x < ex && y >= sy && y < ey) ? 1.f : 0.f;
+// createMask<rect> (src/gpu/cudaConfig.cu:1291-1300): 1 inside [sx,ex) x [sy,ey), and
+// its bits under each pattern's threshold.  A warp writes a word's 32 floats and the word
+// (two kernels, the second reading the first's output back: 12.6 + 18.7 us at 2048^2, now 11.0).
+__global__ void __launch_bounds__(256) k_rect(float* __restrict__ spt, const PatState* __restrict__ stt,
+                                              uint32_t* __restrict__ bits, int rows, int cols, int sx, int sy, int ex,
+                                              int ey) {
+  const int wpr = (cols + 31) >> 5, words = rows * wpr;
+  const int lane = threadIdx.x & 31, nwarp = (gridDim.x * blockDim.x) >> 5;
+  const float thr = stt[blockIdx.y].threshold;
+  float* s = spt + (long long)blockIdx.y * rows * cols;
+  for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < words; w += nwarp) {
+    const int x = w / wpr, y = (w - x * wpr) * 32 + lane;
+    const float v = (x >= sx && x < ex && y >= sy && y < ey) ? 1.f : 0.f;
+    if (y < cols) s[(long long)x * cols + y] = v;
+    const uint32_t b = __ballot_sync(0xffffffffu, y < cols && v > thr);
+    if (lane == 0) bits[(long long)blockIdx.y * words + w] = b;
   }
 }
-cudaError_t rect_support(float* spt, int rows, int cols, int batch, int sx, int sy, int ex, int ey, cudaStream_t st) {
-  k_rect<<<grid1d((long long)rows * cols * batch, 256), 256, 0, st>>>(spt, rows, cols, batch, sx, sy, ex, ey);
+cudaError_t rect_support(float* spt, const PatState* stt, uint32_t* bits, int rows, int cols, int batch, int sx, int sy,
+                         int ex, int ey, cudaStream_t st) {
+  const long long nw = (long long)rows * ((cols + 31) >> 5);
+  const int gx = (int)std::max<long long>(1, std::min<long long>((nw + 7) / 8, std::max(1, sm_count() * 16 / batch)));
+  k_rect<<<dim3(gx, batch), 256, 0, st>>>(spt, stt, bits, rows, cols, sx, sy, ex, ey);
   return cudaGetLastError();
 }
 
 // Support bits: bit = spt > threshold of the pattern (the test of cdi.cu:525).
-// One warp per 32 columns of one row.
-__global__ void k_mask(const float* __restrict__ spt, const PatState* __restrict__ stt, float fixed_thr,
-                       uint32_t* __restrict__ bits, int rows, int cols, int batch) {
-  const int wpr = (cols + 31) >> 5;
-  const long long words = (long long)rows * wpr;
-  const long long nw = words * batch;
-  const int lane = threadIdx.x & 31;
-  for (long long w = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; w < nw;
-       w += ((long long)gridDim.x * blockDim.x) >> 5) {
-    const long long p = w / words, r = (w - p * words) / wpr, cw = (w - p * words) - r * wpr;
-    const int c = (int)cw * 32 + lane;
-    const float thr = stt ? stt[p].threshold : fixed_thr;
-    bool in = false;
-    if (c < cols) in = spt[p * (long long)rows * cols + r * cols + c] > thr;
-    const uint32_t b = __ballot_sync(0xffffffffu, in);
-    if (lane == 0) bits[w] = b;
+// A warp makes four words of a pattern (grid.y) at a time from rows of whole words (cols a
+// multiple of 32: the array is one run of words), else one word of one row.  64-bit
+// divisions per word and one load in flight kept it at 0.9 TB/s (2048^2: 18.7 us, now 4.7).
+__global__ void __launch_bounds__(256) k_mask(const float* __restrict__ spt, const PatState* __restrict__ stt,
+                                              float fixed_thr, uint32_t* __restrict__ bits, int rows, int cols) {
+  const int wpr = (cols + 31) >> 5, words = rows * wpr;
+  const int lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int nwarp = (gridDim.x * blockDim.x) >> 5;
+  const float thr = stt ? stt[blockIdx.y].threshold : fixed_thr;
+  const float* s = spt + (long long)blockIdx.y * rows * cols;
+  uint32_t* o = bits + (long long)blockIdx.y * words;
+  if ((cols & 31) == 0) {
+    for (int w = warp * 4; w < words; w += nwarp * 4) {
+      float v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[k] = w + k < words ? s[(long long)(w + k) * 32 + lane] : 0.f;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint32_t b = __ballot_sync(0xffffffffu, v[k] > thr);
+        if (lane == k && w + k < words) o[w + k] = b;
+      }
+    }
+    return;
+  }
+  for (int w = warp; w < words; w += nwarp) {
+    const int r = w / wpr, c = (w - r * wpr) * 32 + lane;
+    const uint32_t b = __ballot_sync(0xffffffffu, c < cols && s[(long long)r * cols + c] > thr);
+    if (lane == 0) o[w] = b;
   }
 }
 cudaError_t support_bits(const float* spt, const PatState* st_or_null, float fixed_thr, uint32_t* bits, int rows,
                          int cols, int batch, cudaStream_t st) {
-  const long long nw = (long long)rows * ((cols + 31) >> 5) * batch;
-  k_mask<<<grid1d(nw * 32, 256), 256, 0, st>>>(spt, st_or_null, fixed_thr, bits, rows, cols, batch);
+  const long long nw = (long long)rows * ((cols + 31) >> 5);
+  const int gx = (int)std::max<long long>(1, std::min<long long>((nw + 31) / 32, std::max(1, sm_count() * 8 / batch)));
+  k_mask<<<dim3(gx, batch), 256, 0, st>>>(spt, st_or_null, fixed_thr, bits, rows, cols);
   return cudaGetLastError();
 }
 
@@ -350,6 +386,7 @@ cudaError_t shrinkwrap(const float2* rho, float2* tmp, float* spt, const float* 
 __global__ void k_sum_real(const float* __restrict__ x, long long npx, double* __restrict__ part, int nblk) {
   const long long p = blockIdx.y;
   double acc = 0.0;
+#pragma unroll 8
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < npx; i += (long long)nblk * blockDim.x)
     acc += (double)x[p * npx + i];
   __shared__ double red[8];

@@ -9,14 +9,16 @@ cudaError_t scale_complex(float2* x, float s, long long n, cudaStream_t st);
 cudaError_t scale_real(float* x, float s, long long n, cudaStream_t st);
 cudaError_t convert_fo_real(const float* in, float* out, int rows, int cols, int batch, cudaStream_t st);
 cudaError_t convert_fo_complex(const float2* in, float2* out, int rows, int cols, int batch, cudaStream_t st);
-cudaError_t to_tiled(const float* in, float* out, int rows, int cols, int tl, long long out_stride, int batch,
-                     cudaStream_t st);
+// one pattern; amp (may be null) gets sqrt(max(I, 0)) in the same layout
+cudaError_t to_tiled(const float* in, float* out, float* amp, int rows, int cols, int tl, cudaStream_t st);
 cudaError_t mod_abs(float2* psi, const float* inten, long long n, cudaStream_t st);
 cudaError_t mod_ccd(float2* psi, const float* inten, const float* bs, int noise, float scale, float rcolor,
                     long long n, cudaStream_t st);
 cudaError_t apply_support(float2* rho, const float2* rhop, const float* spt, float thr, float beta, int algo,
                           long long n, cudaStream_t st);
-cudaError_t rect_support(float* spt, int rows, int cols, int batch, int sx, int sy, int ex, int ey, cudaStream_t st);
+// the rect support of `batch` patterns and its bits under each pattern's threshold
+cudaError_t rect_support(float* spt, const PatState* stt, uint32_t* bits, int rows, int cols, int batch, int sx, int sy,
+                         int ex, int ey, cudaStream_t st);
 cudaError_t support_bits(const float* spt, const PatState* st_or_null, float fixed_thr, uint32_t* bits, int rows,
                          int cols, int batch, cudaStream_t st);
 // Kernel attributes of the stencil kernels (once per device, outside capture).

@@ -191,7 +191,7 @@ extern "C" int cdx_iterate_noalloc(int rows, int cols, int algo, float beta, int
   // the array keeps the previous call's contents: clear what this call uses
   NA_CK(cudaMemsetAsync(s + o_err, 0, need - o_err, st));
   // sqrt(I), column-tiled (applyModAbs's sqrtf of I > 0, else 0)
-  NA_CK(to_tiled(intensity, amp_t, rows, cols, tl, wst, 1, st));
+  NA_CK(to_tiled(intensity, amp_t, nullptr, rows, cols, tl, st));
   NA_CK(amp_from_pattern(amp_t, amp_t, wst, st));
   // support bits: support > threshold (the test of cdi.cu:525)
   NA_CK(support_bits(support, nullptr, threshold, mask, rows, cols, 1, st));
