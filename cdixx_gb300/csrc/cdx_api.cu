@@ -256,24 +256,26 @@ void plan_shrinkwrap(const cdx_ctx* c, int count, SwPlan& P) {
   }
 }
 
-int col_iter(cdx_ctx* c, bool from_psi, bool rf, float2* psi_proj = nullptr) {
+// One pass of the iteration over the patterns [p0, p0 + nb).
+int col_iter(cdx_ctx* c, int p0, int nb, bool from_psi, bool rf, float2* psi_proj = nullptr) {
   ColArgs a{};
+  const long long to = p0 * c->wstride;
   // the first iteration after a restart reads Psi0 (row-major) from psi
-  a.in = from_psi ? c->psi : c->work;
+  a.in = from_psi ? c->psi + p0 * c->npx : c->work + to;
   a.in_tiled = from_psi ? 0 : 1;
   a.in_stride = from_psi ? c->npx : c->wstride;
-  a.out = c->work;
+  a.out = c->work + to;
   a.out_tiled = 1;
   a.out_stride = c->wstride;
-  a.psi_out = psi_proj;
+  a.psi_out = psi_proj ? psi_proj + p0 * c->npx : nullptr;
   a.psi_stride = c->npx;
-  a.amp = c->amp_t;
-  a.inten = c->inten_t;
-  a.bs = c->bs_t;
+  a.amp = c->amp_t + to;
+  a.inten = c->inten_t + to;
+  a.bs = c->bs_t ? c->bs_t + to : nullptr;
   a.aux_stride = c->wstride;
-  a.state = c->dstate;
+  a.state = c->dstate + p0;
   a.tc = c->p.fft_mode;
-  a.rf_partials = rf ? c->part : nullptr;
+  a.rf_partials = rf ? c->part + (long long)p0 * c->col_blocks : nullptr;
   a.tw = c->tw_r;
   a.cols = c->cols;
   a.mode = COL_ITER;
@@ -286,22 +288,21 @@ int col_iter(cdx_ctx* c, bool from_psi, bool rf, float2* psi_proj = nullptr) {
   a.pdl_mode = c->tune_pdl_col;
   a.err = c->derr;
   a.thin = c->thin;
-  CDX_CK(col_launcher(c->rows)(a, c->batch, c->st));
+  CDX_CK(col_launcher(c->rows)(a, nb, c->st));
   return CDX_OK;
 }
 
-int row_iter(cdx_ctx* c, int algo) {
+int row_iter(cdx_ctx* c, int p0, int nb, int algo) {
   RowArgs a{};
-  a.in = c->work;
-  a.out = c->work;
+  a.in = a.out = c->work + p0 * c->wstride;
   a.in_tiled = a.out_tiled = 1;
   a.tile_log2 = c->tl;
   a.in_stride = a.out_stride = c->wstride;
-  a.rho = c->rho;
+  a.rho = c->rho + p0 * c->npx;
   a.rho_stride = c->npx;
-  a.mask = c->mask;
+  a.mask = c->mask + (long long)p0 * c->rows * c->wpr;
   a.mask_stride = (long long)c->rows * c->wpr;
-  a.state = c->dstate;
+  a.state = c->dstate + p0;
   a.tc = c->p.fft_mode;
   a.tw = c->tw_c;
   a.rows = c->rows;
@@ -314,7 +315,7 @@ int row_iter(cdx_ctx* c, int algo) {
   a.pdl_mode = c->tune_pdl_row;
   a.err = c->derr;
   a.thin = c->thin;
-  CDX_CK(row_launcher(c->cols)(a, c->batch, c->st));
+  CDX_CK(row_launcher(c->cols)(a, nb, c->st));
   return CDX_OK;
 }
 
@@ -353,6 +354,20 @@ int fft2_enqueue(const float2* in, float2* out, int rows, int cols, int batch, b
   return CDX_OK;
 }
 
+// Patterns of a batch the iteration runs on at a time between two shrinkwraps.  An
+// iteration touches rho, W and sqrt(I), 20 bytes a pixel; while those of all patterns
+// fit the L2 (129 MB) the whole batch goes at once, else in equal chunks of up to
+// 100 MB, each for all its iterations, as long as the smallest fills the SMs (us per
+// iteration of the whole batch: 512^2 x48 138.8 -> 127.4, 768^2 x13 92.5 -> 87.8, 1024^2 x8
+// 99 -> 95; 1536^2 x3 as 2 + 1 112.7 -> 117.4, so 3.3 Mpixels are the least).
+int chunk_of(long long npx, long long wstride, int batch) {
+  const double per = 8.0 * npx + 12.0 * wstride, all = per * batch;
+  if (all <= 125e6) return batch;
+  const int chunks = std::min(batch, (int)std::ceil(all / 100e6)), chunk = (batch + chunks - 1) / chunks;
+  const int least = batch - (batch - 1) / chunk * chunk;   // the last chunk
+  return least * npx >= 3300000 ? chunk : batch;
+}
+
 // Enqueue one whole phaseRetrieve on c->st (no synchronisation).
 int enqueue_run(cdx_ctx* c, const std::vector<int>& steps, const SwPlan& sw, bool psi_in_work) {
   const long long n_all = c->npx * c->batch;
@@ -368,7 +383,9 @@ int enqueue_run(cdx_ctx* c, const std::vector<int>& steps, const SwPlan& sw, boo
   const bool prtf = c->pr_map && c->p.prtf_iter >= 0;
   c->pr_reached = false;
   if (prtf) CDX_CK(cudaMemsetAsync(c->pr_map, 0, sizeof(float2) * n_all, c->st));
-  for (int a : steps) {
+  const int chunk = prtf ? c->batch : chunk_of(c->npx, c->wstride, c->batch);
+  for (size_t at = 0; at < steps.size(); ++at) {
+    const int a = steps[at];
     ++step;   // phaseRetrieve's iter: every step, shrinkwraps included
     if (a == ALGO_SHRINKWRAP) {
       const bool m2 = c->p.shrink_mode == CDX_SHRINK_SPATIAL;
@@ -380,15 +397,39 @@ int enqueue_run(cdx_ctx* c, const std::vector<int>& steps, const SwPlan& sw, boo
       ++swi;
       continue;
     }
+    if (chunk < c->batch) {
+      // the iterations up to the next shrinkwrap, a chunk of the patterns at a time
+      size_t end = at;
+      while (end < steps.size() && steps[end] != ALGO_SHRINKWRAP) ++end;
+      const int n = (int)(end - at);
+      for (int p0 = 0; p0 < c->batch; p0 += chunk) {
+        const int nb = std::min(chunk, c->batch - p0);
+        for (int i = 0; i < n; ++i) {
+          const bool rf = c->p.rf_every > 0 && it + i > 0 && ((it + i) % c->p.rf_every) == 0;
+          int e = col_iter(c, p0, nb, from_psi && i == 0, rf);
+          if (e) return e;
+          if (rf)
+            CDX_CK(rfactor_from_partials(c->part + (long long)p0 * c->col_blocks, c->col_blocks, nb, c->dstate + p0,
+                                         c->p.stop_rfactor, it + i, c->p.plateau_iters, c->p.plateau_tol, c->st));
+          if ((e = row_iter(c, p0, nb, steps[at + i]))) return e;
+          nl += rf ? 3 : 2;
+        }
+      }
+      from_psi = false;
+      it += n;
+      step += n - 1;
+      at = end - 1;
+      continue;
+    }
     // from iteration 1 on: the restart iterate has the measured modulus by construction
     const bool rf = c->p.rf_every > 0 && it > 0 && (it % c->p.rf_every) == 0;
     const bool pstep = prtf && step >= c->p.prtf_iter;
-    int e = col_iter(c, from_psi, rf, pstep ? c->pr_psi : nullptr);
+    int e = col_iter(c, 0, c->batch, from_psi, rf, pstep ? c->pr_psi : nullptr);
     if (e) return e;
     if (rf)
       CDX_CK(rfactor_from_partials(c->part, c->col_blocks, c->batch, c->dstate, c->p.stop_rfactor, it,
                                    c->p.plateau_iters, c->p.plateau_tol, c->st));
-    e = row_iter(c, a);
+    e = row_iter(c, 0, c->batch, a);
     if (e) return e;
     nl += rf ? 3 : 2;
     if (pstep) {
@@ -566,8 +607,8 @@ int autotune(cdx_ctx* c) {
         cudaGraphExec_t ge = nullptr;
         CDX_CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
         for (int i = 0; i < kTimed && e == CDX_OK; ++i) {
-          e = col_iter(c, false, false);
-          if (e == CDX_OK) e = row_iter(c, ALGO_HIO);
+          e = col_iter(c, 0, c->batch, false, false);
+          if (e == CDX_OK) e = row_iter(c, 0, c->batch, ALGO_HIO);
         }
         const cudaError_t ce = cudaStreamEndCapture(c->st, &g);
         if (e == CDX_OK && ce != cudaSuccess) e = set_error(CDX_ERR_CUDA, std::string("autotune capture: ") + cudaGetErrorString(ce));
