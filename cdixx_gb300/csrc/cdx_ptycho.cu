@@ -324,24 +324,11 @@ __global__ void k_pty_csum(const float2* __restrict__ O, const float* __restrict
                            PtyScal* s, unsigned* count, int final_phase) {
   __shared__ double red[2][8];
   float ax = 0.f, ay = 0.f;
-  // sixteen loads in flight per thread; the sum's order is that of a plain loop
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += 16 * stride) {
-    float2 v[16];
-    float f[16];
-#pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      const long long j = i + u * stride;
-      v[u] = j < n ? O[j] : make_float2(0.f, 0.f);
-      f[u] = m && j < n ? m[j] : 1.f;
-    }
-#pragma unroll
-    for (int u = 0; u < 16; ++u) {
-      if (i + u * stride >= n) break;
-      if (m) { v[u].x *= f[u]; v[u].y *= f[u]; }
-      ax += v[u].x;
-      ay += v[u].y;
-    }
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    float2 v = O[i];
+    if (m) { const float f = m[i]; v.x *= f; v.y *= f; }
+    ax += v.x;
+    ay += v.y;
   }
   double sx = ax, sy = ay;
   for (int o = 16; o; o >>= 1) {
