@@ -81,6 +81,12 @@ int check_len(int n) {
 
 }  // namespace
 
+// What a run brings back to the host, in pinned memory: one wait covers both copies.
+struct RunBack {
+  int err;
+  PatState state;
+};
+
 struct cdx_ctx {
   cdx_params p{};
   int rows = 0, cols = 0, batch = 0;
@@ -107,6 +113,7 @@ struct cdx_ctx {
   PatState* dstate = nullptr;
   float* weights = nullptr;
   size_t weights_cap = 0;
+  std::vector<float> weights_host;   // what `weights` holds
   void* arena = nullptr;
   size_t arena_bytes = 0;
 
@@ -130,6 +137,7 @@ struct cdx_ctx {
   // launch variant (autotune): RowArgs/ColArgs knobs, and what was measured
   int tune_pdl_col = 0, tune_pdl_row = 0, tune_cb_plus1 = 0;   // pdl: 0 per-length default, 1 plain, 2 PDL
   int* derr = nullptr;        // bulk-copy wait timeouts of the pass kernels (bit 0)
+  RunBack* back = nullptr;
   bool tuned = false;
   std::string tune_report;
 
@@ -508,11 +516,16 @@ int prepare_run(cdx_ctx* c, const char* algorithm, std::vector<int>& steps, SwPl
       if (c->weights) cudaFree(c->weights);
       c->weights = nullptr;
       c->weights_cap = 0;
+      c->weights_host.clear();
       CDX_CK(cudaMalloc(&c->weights, sizeof(float) * sw.w.size()));
       c->weights_cap = sw.w.size();
     }
-    CDX_CK(cudaMemcpyAsync(c->weights, sw.w.data(), sizeof(float) * sw.w.size(), cudaMemcpyHostToDevice, c->st));
-    CDX_CK(cudaStreamSynchronize(c->st));
+    if (sw.w != c->weights_host) {   // else the last run's schedule is there already
+      c->weights_host.clear();
+      CDX_CK(cudaMemcpyAsync(c->weights, sw.w.data(), sizeof(float) * sw.w.size(), cudaMemcpyHostToDevice, c->st));
+      CDX_CK(cudaStreamSynchronize(c->st));
+      c->weights_host = sw.w;
+    }
   }
   c->last_steps = (int)steps.size();
   c->last_sw = nsw;
@@ -868,11 +881,9 @@ int group_run_impl(cdx_group* g, const char* algorithm, double* gpu_ms) {
   return CDX_OK;
 }
 
-int fill_stats(cdx_ctx* c, int idx, cdx_stats* s) {
-  if (!s) return CDX_OK;
-  PatState h;
-  CDX_CK(cudaMemcpyAsync(&h, c->dstate + idx, sizeof h, cudaMemcpyDeviceToHost, c->st));
-  CDX_CK(cudaStreamSynchronize(c->st));
+// The statistics of the pattern whose state c->back holds.
+int stats_of_back(cdx_ctx* c, cdx_stats* s) {
+  const PatState& h = c->back->state;
   memset(s, 0, sizeof *s);
   s->steps = c->last_steps;
   s->iterations = c->last_iters;
@@ -888,6 +899,13 @@ int fill_stats(cdx_ctx* c, int idx, cdx_stats* s) {
   if (cudaEventElapsedTime(&ms, c->ev0, c->ev1) == cudaSuccess) s->gpu_ms = ms;
   else cudaGetLastError();
   return CDX_OK;
+}
+
+int fill_stats(cdx_ctx* c, int idx, cdx_stats* s) {
+  if (!s) return CDX_OK;
+  CDX_CK(cudaMemcpyAsync(&c->back->state, c->dstate + idx, sizeof(PatState), cudaMemcpyDeviceToHost, c->st));
+  CDX_CK(cudaStreamSynchronize(c->st));
+  return stats_of_back(c, s);
 }
 
 }  // namespace
@@ -1031,6 +1049,8 @@ int cdx_create(const cdx_params* p, void* stream, cdx_ctx** out) {
          cudaMemsetAsync(c->pr_state, 0, sizeof(PrtfState) * c->batch, c->st) == cudaSuccess;
     if (!ok) return fail(set_error(CDX_ERR_CUDA, "PRTF buffer clear"));
   }
+  if (cudaHostAlloc(&c->back, sizeof(RunBack), cudaHostAllocDefault) != cudaSuccess)
+    return fail(set_error(CDX_ERR_NOMEM, "pinned run statistics"));
   if (cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess)
     return fail(set_error(CDX_ERR_CUDA, "event create failed"));
   if (cudaStreamSynchronize(c->st) != cudaSuccess)
@@ -1050,6 +1070,7 @@ int cdx_destroy(cdx_ctx* c) {
   for (void* q : {(void*)c->pr_psi, (void*)c->pr_rhop, (void*)c->pr_cache, (void*)c->pr_gamma0, (void*)c->pr_map,
                   (void*)c->pr_mask, (void*)c->pr_polar, (void*)c->pr_part, (void*)c->pr_state})
     if (q) cudaFree(q);
+  if (c->back) cudaFreeHost(c->back);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
   if (c->own_stream && c->st) cudaStreamDestroy(c->st);
@@ -1300,24 +1321,19 @@ int cdx_group_destroy(cdx_group* g) {
   return CDX_OK;
 }
 
-// A pass kernel whose staging copy did not complete within its bounded wait
-// leaves bit 0 in the context's error word; reported (and cleared) here.
-int check_bulk(cdx_ctx* c) {
-  int h = 0;
-  CDX_CK(cudaMemcpy(&h, c->derr, sizeof(int), cudaMemcpyDeviceToHost));
-  if (h) {
-    CDX_CK(cudaMemset(c->derr, 0, sizeof(int)));
-    return set_error(CDX_ERR_CUDA, "a pass kernel's bulk staging copy timed out; the run's results are invalid");
-  }
-  return CDX_OK;
-}
-
 int cdx_run(cdx_ctx* c, const char* algorithm, cdx_stats* stats) {
   int e = run_impl(c, algorithm);
   if (e) return e;
+  CDX_CK(cudaMemcpyAsync(&c->back->err, c->derr, sizeof(int), cudaMemcpyDeviceToHost, c->st));
+  CDX_CK(cudaMemcpyAsync(&c->back->state, c->dstate, sizeof(PatState), cudaMemcpyDeviceToHost, c->st));
   CDX_CK(cudaStreamSynchronize(c->st));
-  if ((e = check_bulk(c))) return e;
-  return fill_stats(c, 0, stats);
+  // a pass kernel whose staging copy did not complete within its bounded wait leaves bit 0 in
+  // the context's error word; reported and cleared here
+  if (c->back->err) {
+    CDX_CK(cudaMemset(c->derr, 0, sizeof(int)));
+    return set_error(CDX_ERR_CUDA, "a pass kernel's bulk staging copy timed out; the run's results are invalid");
+  }
+  return stats ? stats_of_back(c, stats) : CDX_OK;
 }
 
 int cdx_get_stats(cdx_ctx* c, int idx, cdx_stats* s) {
