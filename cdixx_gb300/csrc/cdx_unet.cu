@@ -41,26 +41,27 @@ constexpr int kThreads = 256;
 // unsigned order is float order): one slice of a pattern per CTA, so that a few
 // patterns still use every SM (one CTA per pattern took 174 us for 8 of 256^2).
 __global__ void k_prep_max(const float* __restrict__ inten, int P, unsigned* __restrict__ mx) {
-  const float* I = inten + (long long)blockIdx.y * P;
+  const float* I = inten + (long long)blockIdx.x * P;
   float m = 0.f;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < P; i += gridDim.x * blockDim.x)
+  for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < P; i += gridDim.y * blockDim.x)
     m = fmaxf(m, log1pf(fmaxf(I[i], 0.f)));
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) atomicMax(mx + blockIdx.y, __float_as_uint(m));
+  if ((threadIdx.x & 31) == 0) atomicMax(mx + blockIdx.x, __float_as_uint(m));
 }
 // log(1 + I) / max log(1 + I) per pattern, centred (fftshift), channel 0 of 8 (one 16-byte store)
 __global__ void k_prep_input(const float* __restrict__ inten, const unsigned* __restrict__ mx,
                              __nv_bfloat16* __restrict__ x, int n) {
+  net_wait();
   const int P = n * n, h = n / 2;
-  const float* I = inten + (long long)blockIdx.y * P;
-  const float top = __uint_as_float(mx[blockIdx.y]);
+  const float* I = inten + (long long)blockIdx.x * P;
+  const float top = __uint_as_float(mx[blockIdx.x]);
   const float inv = top > 0.f ? 1.f / top : 0.f;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < P; i += gridDim.x * blockDim.x) {
+  for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < P; i += gridDim.y * blockDim.x) {
     const int y = i / n, xx = i - y * n;
     const int sy = y < h ? y + h : y - h, sx = xx < h ? xx + h : xx - h;   // centred pixel <- FFT-order pixel
     const float v = log1pf(fmaxf(I[sy * n + sx], 0.f)) * inv;
     const __nv_bfloat162 b = __halves2bfloat162(__float2bfloat16(v), __float2bfloat16(0.f));
-    reinterpret_cast<uint4*>(x)[(long long)blockIdx.y * P + i] =
+    reinterpret_cast<uint4*>(x)[(long long)blockIdx.x * P + i] =
         make_uint4(*reinterpret_cast<const unsigned*>(&b), 0u, 0u, 0u);
   }
 }
@@ -131,6 +132,7 @@ __device__ __forceinline__ void gn_tree(double* r, int gpc, int stop) {
 // statistics: partial sums per (pattern, group, split); grid (patterns, split, G / gpc)
 __global__ void __launch_bounds__(512) k_gn_stats(const float* __restrict__ x, int HW, int C, int G, int gpc,
                                                   int split, double* __restrict__ part) {
+  net_wait();
   const int n = blockIdx.x, z = blockIdx.y, Cg = C / G, kc = gpc * Cg, tpc = kThreads / Cg;
   const int q4 = kc / 4, q = threadIdx.x % q4, p0 = threadIdx.x / q4;
   const int pb = (int)((long long)HW * z / split), pe = (int)((long long)HW * (z + 1) / split);
@@ -182,8 +184,8 @@ __global__ void __launch_bounds__(512) k_gn_stats(const float* __restrict__ x, i
   }
 }
 
-// Element-wise GroupNorm kernels: a CTA takes a range of pixels of one pattern
-// (grid.y) and, a thread each, eight channels of a pixel; octets beyond 256 go to
+// Element-wise GroupNorm kernels: a CTA takes a range of pixels (grid.y) of one pattern
+// (grid.x) and, a thread each, eight channels of a pixel; octets beyond 256 go to
 // grid.z.  A thread keeps its channels over the range, so the per-channel values
 // stay in registers.
 struct GnSpan {
@@ -198,8 +200,8 @@ __device__ __forceinline__ GnSpan gn_span(int HW, int C) {
   s.oct = blockIdx.z * oc + threadIdx.x % oc;
   const int r = threadIdx.x / oc;
   s.ok = r < s.step && s.oct < C / 8;
-  s.p = (int)((long long)HW * blockIdx.x / gridDim.x) + r;
-  s.pe = (int)((long long)HW * (blockIdx.x + 1) / gridDim.x);
+  s.p = (int)((long long)HW * blockIdx.y / gridDim.y) + r;
+  s.pe = (int)((long long)HW * (blockIdx.y + 1) / gridDim.y);
   return s;
 }
 __device__ __forceinline__ void ld8(float (&v)[8], const float* p) {
@@ -222,7 +224,8 @@ __global__ void __launch_bounds__(kThreads) k_gn_apply(const float* __restrict__
                                                        const float* __restrict__ gamma, const float* __restrict__ beta,
                                                        int HW, int C, int G, float slope, __nv_bfloat16* __restrict__ y) {
   extern __shared__ float2 st[];   // mean, rstd per group
-  const int n = blockIdx.y, Cg = C / G;
+  net_wait();
+  const int n = blockIdx.x, Cg = C / G;
   for (int g = threadIdx.x; g < G; g += kThreads) {
     double s = 0.0, q = 0.0;
 #pragma unroll 8
@@ -235,7 +238,7 @@ __global__ void __launch_bounds__(kThreads) k_gn_apply(const float* __restrict__
     const double mean = s / count;
     const double var = fmax(q / count - mean * mean, 0.0);
     st[g] = make_float2((float)mean, (float)(1.0 / sqrt(var + 1e-5)));
-    if (blockIdx.x == 0 && blockIdx.z == 0) reinterpret_cast<float2*>(stats)[n * G + g] = st[g];
+    if (blockIdx.y == 0 && blockIdx.z == 0) reinterpret_cast<float2*>(stats)[n * G + g] = st[g];
   }
   __syncthreads();
   const GnSpan t = gn_span(HW, C);
@@ -379,7 +382,7 @@ __global__ void __launch_bounds__(kThreads) k_gn_bwd_apply(const float* __restri
                                                            int HW, int C, int G, float slope,
                                                            __nv_bfloat16* __restrict__ dx) {
   extern __shared__ float4 sg[];   // mean, rstd, S1, S2 per group
-  const int n = blockIdx.y, Cg = C / G;
+  const int n = blockIdx.x, Cg = C / G;
   const float inv_m = 1.f / ((float)HW * Cg);
   for (int g = threadIdx.x; g < G; g += kThreads) {
     const long long ng = (long long)n * G + g;
@@ -674,6 +677,7 @@ struct Net {
   float2* wrk = nullptr;   // warm start scratch
   int* umma_err = nullptr; // set by a tcgen05 tile whose pipeline wait timed out
   int adam_t = 0;
+  bool dep = false;        // launch the forward's kernels dependently (small passes)
   bool weights_dirty = true;
 };
 
@@ -883,7 +887,7 @@ int launch_gemm(const Net* u, const GemmArgs& a, const __nv_bfloat16* packed, cu
   ConvUmma c;
   int smem = 0;
   if (plan_umma<DGRAD>(a, packed, c, smem)) {
-    U_CK(launch_conv_umma(c, smem, u->umma_err, st));
+    U_CK(launch_conv_umma(c, smem, u->umma_err, u->dep, st));
     return CDX_OK;
   }
   const long long M = DGRAD ? (long long)s.N * s.H * s.W : (long long)s.N * s.Ho * s.Wo;
@@ -897,9 +901,7 @@ int launch_gemm(const Net* u, const GemmArgs& a, const __nv_bfloat16* packed, cu
     return launch_umma<128>(op, M, NC, K, u->umma_err, st);
   }
   const dim3 grid((unsigned)((M + 127) / 128), (unsigned)((NC + (NC <= 32 ? 31 : 63)) / (NC <= 32 ? 32 : 64)));
-  if (NC <= 32) k_conv_gemm<DGRAD, 32><<<grid, 128, 0, st>>>(a);
-  else k_conv_gemm<DGRAD, 64><<<grid, 128, 0, st>>>(a);
-  U_CK(cudaGetLastError());
+  U_CK(net_launch(u->dep, NC <= 32 ? k_conv_gemm<DGRAD, 32> : k_conv_gemm<DGRAD, 64>, grid, 128, 0, st, a));
   return CDX_OK;
 }
 
@@ -943,18 +945,19 @@ int gn_split(const Net* u, int HW, int count) {
 dim3 gn_grid(int HW, int C, int count) {
   const int oc = gn_octs(C), per = kThreads / oc * 4;
   const int x = std::max(1, std::min((HW + per - 1) / per, sm_count() * 8 / count));
-  return dim3(x, count, (C / 8 + oc - 1) / oc);
+  return dim3(count, x, (C / 8 + oc - 1) / oc);
 }
 
 int forward(Net* u, const float* inten, int count) {
   const cdx_unet_config& c = u->cfg;
   int e = refresh_weights(u);
   if (e) return e;
+  u->dep = (long long)count * c.n * c.n <= 1LL << 20;
   U_CK(cudaMemsetAsync(u->mx, 0, sizeof(unsigned) * count, u->st));
   const int P = c.n * c.n;
-  const dim3 pgrid(std::max(1, std::min((P + kThreads - 1) / kThreads, sm_count() * 8 / count)), count);
+  const dim3 pgrid(count, std::max(1, std::min((P + kThreads - 1) / kThreads, sm_count() * 8 / count)));
   k_prep_max<<<pgrid, kThreads, 0, u->st>>>(inten, P, u->mx);
-  k_prep_input<<<pgrid, kThreads, 0, u->st>>>(inten, u->mx, u->x_in, c.n);
+  U_CK(net_launch(u->dep, k_prep_input, pgrid, kThreads, 0, u->st, inten, u->mx, u->x_in, c.n));
   for (auto& l : u->L) {
     GemmArgs a{};
     a.s = conv_shape(u, l, count);
@@ -977,10 +980,10 @@ int forward(Net* u, const float* inten, int count) {
       continue;
     }
     const int HW = l.out_h * l.out_h, sp = gn_split(u, HW, count), C = l.cout_p, gpc = gn_groups(C / c.groups, c.groups);
-    k_gn_stats<<<dim3(count, sp, c.groups / gpc), kThreads / 4 * gpc, gpc * kThreads * sizeof(double), u->st>>>(
-        l.pre, HW, C, c.groups, gpc, sp, u->gpart);
-    k_gn_apply<<<gn_grid(HW, C, count), kThreads, c.groups * sizeof(float2), u->st>>>(
-        l.pre, u->gpart, sp, l.stats, u->params + l.g_off, u->params + l.b_off, HW, C, c.groups, c.slope, l.act);
+    U_CK(net_launch(u->dep, k_gn_stats, dim3(count, sp, c.groups / gpc), kThreads / 4 * gpc, gpc * kThreads * sizeof(double),
+                    u->st, l.pre, HW, C, c.groups, gpc, sp, u->gpart));
+    U_CK(net_launch(u->dep, k_gn_apply, gn_grid(HW, C, count), kThreads, c.groups * sizeof(float2), u->st, l.pre, u->gpart, sp,
+                    l.stats, u->params + l.g_off, u->params + l.b_off, HW, C, c.groups, c.slope, l.act));
   }
   U_CK(cudaGetLastError());
   return CDX_OK;
@@ -990,6 +993,7 @@ int backward(Net* u, const float* amp_t, const float* ph_t, const float* sup_t, 
   const cdx_unet_config& c = u->cfg;
   const Layer& head = u->L.back();
   const int P = c.n * c.n;
+  u->dep = false;
   // the first data gradient that reaches a layer's activation is stored, later ones are added
   std::vector<char> reached(u->L.size(), 0);
   const int lsp = std::max(1, std::min(64, (sm_count() * 4 + count - 1) / count));
@@ -1117,6 +1121,10 @@ int cdx_unet_create(const cdx_unet_config* c, void* stream, cdx_unet** out) {
     n->own_stream = true;
   }
   int e = build(n);
+  // the element-wise GroupNorm kernels hold a pattern's group statistics (16 bytes a group at most)
+  for (const void* k : {(const void*)k_gn_apply, (const void*)k_gn_bwd_apply})
+    if (!e && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess)
+      e = set_error(CDX_ERR_CUDA, "kernel attributes");
   if (!e) {
     std::vector<float> h;
     init_params(n, h);

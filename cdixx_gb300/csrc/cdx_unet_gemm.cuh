@@ -71,6 +71,30 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// Programmatic dependent launch (dep) of the network's kernels: each first waits for the one
+// before it (which waited for the one before that) and lets the next be scheduled, so a
+// launch's latency and set-up pass behind the tail of its predecessor.  For small forward
+// passes (8 patterns of 256^2: 1109 -> 1072 us); in a training step of 32 the early CTAs took
+// the running kernel's room (10.9 -> 11.4 ms), so large passes and the backward launch plainly.
+__device__ __forceinline__ void net_wait() {
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+template <class... P, class... A>
+cudaError_t net_launch(bool dep, void (*kernel)(P...), dim3 grid, int block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = dep ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // byte offset of 16-byte chunk c of row r in a tile with 64-byte rows
 __device__ __forceinline__ int sw64(int r, int c) { return r * 64 + ((c ^ ((r >> 1) & 3)) << 4); }
 // ... with 128-byte rows
@@ -118,6 +142,7 @@ __global__ void __launch_bounds__(128) k_conv_gemm(GemmArgs a) {
   const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wm = warp >> 1, wn = warp & 1;
+  net_wait();
 
   // this thread stages row `tid` of the A tile: decode its pixel once
   const int am = m0 + tid;

@@ -26,6 +26,7 @@
 // 256^2 (4 levels, 32 channels): the step's 26 launches take 2.7 ms (10.5 with the
 // gathering kernels), the network on 8 patterns 1.91 -> 1.11 ms as a whole.
 #pragma once
+#include "cdx_unet_gemm.cuh"
 #include "cdx_umma.cuh"
 
 namespace cdx {
@@ -105,6 +106,7 @@ __global__ void __launch_bounds__(kCuThreads, 3) k_conv_umma(const __grid_consta
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  net_wait();   // the barriers and TMEM are set up behind the predecessor's tail
   const unsigned tmem = tmem_base;
   auto give_up = [&]() {
     abort_flag = 1;
@@ -338,7 +340,7 @@ inline bool cu_plan(ConvUmma& a, int taps, int& smem) {
   return a.nstage >= 2;
 }
 
-inline cudaError_t launch_conv_umma(const ConvUmma& a, int smem, int* err, cudaStream_t st) {
+inline cudaError_t launch_conv_umma(const ConvUmma& a, int smem, int* err, bool dep, cudaStream_t st) {
   static std::atomic<unsigned long long> done{0};   // attribute set, bit per device
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -355,8 +357,7 @@ inline cudaError_t launch_conv_umma(const ConvUmma& a, int smem, int* err, cudaS
   const int per_sm = std::max(1, std::min({(228 * 1024) / (smem + 1024 + 11 * 1024), 512 / cols, 3}));
   const long long tiles = (long long)a.nimg * ((a.GH + kCuTH - 1) / kCuTH) * ((a.GW + kCuTW - 1) / kCuTW);
   const int grid = (int)std::min<long long>(tiles, (long long)per_sm * sm_count());
-  k_conv_umma<<<grid, kCuThreads, smem, st>>>(a, err);
-  return cudaGetLastError();
+  return net_launch(dep, k_conv_umma, grid, kCuThreads, smem, st, a, err);
 }
 
 // Geometry of the five forms.  3x3 stride 1 (flip: the data gradient's taps run the other way).
