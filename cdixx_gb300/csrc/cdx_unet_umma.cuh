@@ -22,9 +22,12 @@
 // (two, in TMEM), warp 8 issues the MMAs, warp 9 the weight copies.  Every wait is
 // bounded; a role that gives up sets *err and the abort flag, which ends the others.
 //
-// Bound by HBM and the L2 (FP32 outputs, patches and streamed weights).  Batch 32 of
-// 256^2 (4 levels, 32 channels): the step's 26 launches take 2.7 ms (10.5 with the
-// gathering kernels), the network on 8 patterns 1.91 -> 1.11 ms as a whole.
+// Bound by HBM and the L2 (FP32 outputs, patches and streamed weights), and before that by
+// the MMA lane: one thread issues every MMA, and a loop that builds both descriptors
+// each time spent 130-190 cycles per MMA on it.  The loops below add to descriptors
+// built once and are unrolled: batch 32 of 256^2 (4 levels, 32 channels), the step's 26
+// launches 3.02 -> 2.60 ms (10.5 with the gathering kernels), 32 -> 32 channels at 256^2
+// 113 -> 91 us; the network on 8 patterns 1.08 -> 1.03 ms as a whole.
 #pragma once
 #include "cdx_unet_gemm.cuh"
 #include "cdx_umma.cuh"
@@ -235,27 +238,31 @@ __global__ void __launch_bounds__(kCuThreads, 3) k_conv_umma(const __grid_consta
           }
           asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
           const unsigned d = tmem + (unsigned)(ab * N);
-          int accum = 0;
-          for (int i = 0; i < a.ntap[cls] && !failed; ++i) {
-            const unsigned at = pa + (unsigned)a.aoff[cls][i] * 16;
-            for (int k = 0; k < chunks; ++k) {
-              unsigned wa;
-              if (a.nstage) {
+          // a 16-byte step of an operand's start is one more in its descriptor
+          const uint64_t da = cu_desc(pa, plane, sbo);
+          const unsigned as = 2 * plane >> 4, ws = 2 * wcol >> 4;
+          if (a.nstage == 0) {
+            const uint64_t dw = cu_desc(weights, wcol, 128);
+            const int steps = a.C >> 4;
+#pragma unroll 3
+            for (int i = 0; i < a.ntap[cls]; ++i) {
+              const uint64_t di = da + a.aoff[cls][i], dt = dw + (unsigned)a.tap[cls][i] * steps * ws;
+#pragma unroll 2
+              for (int kk = 0; kk < steps; ++kk) mma_f16(d, di + kk * as, dt + kk * ws, idesc, i > 0 || kk > 0);
+            }
+          } else {
+            for (int i = 0; i < a.ntap[cls] && !failed; ++i) {
+              const uint64_t di = da + a.aoff[cls][i];
+              for (int k = 0; k < chunks; ++k) {
                 if (!mbar_wait_or_abort(smem_u32(&wfull[s]), sp, &abort_flag)) {
                   failed = true;
                   break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                wa = weights + s * stage_bytes;
-              } else {
-                wa = weights + (unsigned)a.tap[cls][i] * C8 * wcol;
-              }
-              const int k0 = a.nstage ? k * spc : 0, k1 = a.nstage ? min(k0 + spc, a.C >> 4) : a.C >> 4;
-              for (int kk = k0; kk < k1; ++kk, wa += 2 * wcol) {
-                mma_f16(d, cu_desc(at + kk * 2 * plane, plane, sbo), cu_desc(wa, wcol, 128), idesc, accum);
-                accum = 1;
-              }
-              if (a.nstage) {
+                const uint64_t dw = cu_desc(weights + s * stage_bytes, wcol, 128), dk = di + k * spc * as;
+                const int steps = min(spc, (a.C >> 4) - k * spc);
+#pragma unroll 8
+                for (int kk = 0; kk < steps; ++kk) mma_f16(d, dk + kk * as, dw + kk * ws, idesc, i > 0 || k > 0 || kk > 0);
                 mma_commit(smem_u32(&wempty[s]));
                 if (++s == a.nstage) { s = 0; sp ^= 1; }
               }
@@ -430,8 +437,10 @@ inline void cu_adj_s2(ConvUmma& a, int k, int p) {
 // split of the pixels, which it walks in order in steps of 16, as k_conv_wgrad does:
 // the partial sums are the same, bit for bit.  Rows of M and columns of N past the
 // channels multiply whatever lies behind the planes and are not read back.
-// Bound by the operands' reads from shared memory (an MMA of M = 128 takes 32 cycles
-// whatever N up to 64).  Batch 32 of 256^2: the step's 15 launches 8.5 -> 3.9 ms.
+// Bound by the chain of MMAs of a CTA (a split's pixels in order) and by the lane that
+// issues them.  Batch 32 of 256^2: the step's 15 launches 8.5 -> 3.9 ms, and 2.9 with
+// descriptors added to and the loop unrolled (32 -> 32 channels at 256^2 576 -> 350 us, the
+// 1x1 head 306 -> 138; unrolled by 4 and by 8 1-2 % apart).
 constexpr int kWgStages = 4, kWgAhead = 2;
 constexpr int kWgThreads = 160;     // warps 0-3 copy and then drain the accumulators, warp 4 issues the MMAs
 
@@ -579,12 +588,21 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_wgrad_umma(const __grid_const
         }
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         const unsigned xa = base + s * a.stage, ya = xa + a.xpl * xplane;
-        for (int p = 0; p < len; p += 16)
-          for (int t = 0; t < a.KW; ++t) {
-            const int slot = a.S == 1 ? p + t : (t & 1) * par + p + (t >> 1);
-            const uint64_t dx = wg_desc(xa + slot * 16, xplane), dy = wg_desc(ya + p * 16, yplane);
-            mma_f16(tmem + t * ncol, a.m_is_x ? dx : dy, a.m_is_x ? dy : dx, idesc, g > 0 || p > 0);
-          }
+        const uint64_t dx = wg_desc(xa, xplane), dy = wg_desc(ya, yplane);   // a slot further is one more
+        auto steps = [&](auto kw) {
+          constexpr int KW = decltype(kw)::value;
+          const uint64_t dm = a.m_is_x ? dx : dy, dn = a.m_is_x ? dy : dx;
+#pragma unroll 8
+          for (int p = 0; p < len; p += 16)
+#pragma unroll
+            for (int t = 0; t < KW; ++t) {
+              const int off = a.S == 1 ? t : (t & 1) * par + (t >> 1);
+              mma_f16(tmem + t * ncol, dm + p + (a.m_is_x ? off : 0), dn + p + (a.m_is_x ? 0 : off), idesc, g > 0 || p > 0);
+            }
+        };
+        if (a.KW == 3) steps(std::integral_constant<int, 3>());
+        else if (a.KW == 2) steps(std::integral_constant<int, 2>());
+        else steps(std::integral_constant<int, 1>());
         mma_commit(smem_u32(&empty[s]));
         m += len;
       }
