@@ -133,6 +133,7 @@ struct cdx_ctx {
   PrtfState* pr_state = nullptr;
   bool pr_valid = false;       // the last run reached prtf_iter
   bool pr_reached = false;     // set while enqueueing
+  bool own_stops = false;      // a pattern was given a stop of its own
 
   // launch variant (autotune): RowArgs/ColArgs knobs, and what was measured
   int tune_pdl_col = 0, tune_pdl_row = 0, tune_cb_plus1 = 0;   // pdl: 0 per-length default, 1 plain, 2 PDL
@@ -362,18 +363,19 @@ int fft2_enqueue(const float2* in, float2* out, int rows, int cols, int batch, b
   return CDX_OK;
 }
 
-// Patterns of a batch the iteration runs on at a time between two shrinkwraps.  An
-// iteration touches rho, W and sqrt(I), 20 bytes a pixel; while those of all patterns
-// fit the L2 (129 MB) the whole batch goes at once, else in equal chunks of up to
-// 100 MB, each for all its iterations, as long as the smallest fills the SMs (us per
-// iteration of the whole batch: 512^2 x48 138.8 -> 127.4, 768^2 x13 92.5 -> 87.8, 1024^2 x8
-// 99 -> 95; 1536^2 x3 as 2 + 1 112.7 -> 117.4, so 3.3 Mpixels are the least).
-int chunk_of(long long npx, long long wstride, int batch) {
-  const double per = 8.0 * npx + 12.0 * wstride, all = per * batch;
-  if (all <= 125e6) return batch;
-  const int chunks = std::min(batch, (int)std::ceil(all / 100e6)), chunk = (batch + chunks - 1) / chunks;
-  const int least = batch - (batch - 1) / chunk * chunk;   // the last chunk
-  return least * npx >= 3300000 ? chunk : batch;
+// Chunks a batch iterates in between two shrinkwraps.  An iteration touches rho, W and
+// sqrt(I), 20 bytes a pixel; while those of all patterns fit the L2 (129 MB) the whole
+// batch goes at once, else in even chunks of up to 100 MB, each for all its iterations, as
+// long as the smallest fills the SMs (us per iteration of the whole batch: 512^2 x48 138.8
+// -> 127.4, 768^2 x13 92.5 -> 87.8, 1024^2 x8 99 -> 95; 1536^2 x3 as 2 + 1 112.7 -> 117.4, so
+// 3.3 Mpixels are the least).  Runs whose patterns may stop stay whole: once most have
+// stopped, chunks are many small launches (1024 of 256^2 to an R plateau, 2000 iterations:
+// 754 ms in chunks, 697 whole; 256 of 512^2 to stops of their own 1329, 1246).
+int chunks_of(long long npx, long long wstride, int batch, bool stops) {
+  const double all = (8.0 * npx + 12.0 * wstride) * batch;
+  if (all <= 125e6 || stops) return 1;
+  const int chunks = std::min(batch, (int)std::ceil(all / 100e6));
+  return batch / chunks * npx >= 3300000 ? chunks : 1;
 }
 
 // Enqueue one whole phaseRetrieve on c->st (no synchronisation).
@@ -391,7 +393,8 @@ int enqueue_run(cdx_ctx* c, const std::vector<int>& steps, const SwPlan& sw, boo
   const bool prtf = c->pr_map && c->p.prtf_iter >= 0;
   c->pr_reached = false;
   if (prtf) CDX_CK(cudaMemsetAsync(c->pr_map, 0, sizeof(float2) * n_all, c->st));
-  const int chunk = prtf ? c->batch : chunk_of(c->npx, c->wstride, c->batch);
+  const bool stops = c->p.rf_every > 0 && (c->p.stop_rfactor > 0 || c->p.plateau_iters > 0 || c->own_stops);
+  const int chunks = prtf ? 1 : chunks_of(c->npx, c->wstride, c->batch, stops);
   for (size_t at = 0; at < steps.size(); ++at) {
     const int a = steps[at];
     ++step;   // phaseRetrieve's iter: every step, shrinkwraps included
@@ -405,13 +408,13 @@ int enqueue_run(cdx_ctx* c, const std::vector<int>& steps, const SwPlan& sw, boo
       ++swi;
       continue;
     }
-    if (chunk < c->batch) {
+    if (chunks > 1) {
       // the iterations up to the next shrinkwrap, a chunk of the patterns at a time
       size_t end = at;
       while (end < steps.size() && steps[end] != ALGO_SHRINKWRAP) ++end;
       const int n = (int)(end - at);
-      for (int p0 = 0; p0 < c->batch; p0 += chunk) {
-        const int nb = std::min(chunk, c->batch - p0);
+      for (int k = 0, p0 = 0, nb; k < chunks; ++k, p0 += nb) {
+        nb = c->batch / chunks + (k < c->batch % chunks);
         for (int i = 0; i < n; ++i) {
           const bool rf = c->p.rf_every > 0 && it + i > 0 && ((it + i) % c->p.rf_every) == 0;
           int e = col_iter(c, p0, nb, from_psi && i == 0, rf);
@@ -1266,6 +1269,7 @@ int cdx_set_support(cdx_ctx* c, int idx, const float* support, int where) {
 
 int cdx_set_stop_rfactor(cdx_ctx* c, int idx, double stop) {
   if (!c || idx < 0 || idx >= c->batch || !(stop >= 0.0)) return set_error(CDX_ERR_ARG, "bad stop argument");
+  c->own_stops = c->own_stops || stop > 0;
   CDX_CK(cudaMemcpyAsync(&c->dstate[idx].stop, &stop, sizeof(double), cudaMemcpyHostToDevice, c->st));
   CDX_CK(cudaStreamSynchronize(c->st));
   return CDX_OK;
