@@ -16,6 +16,7 @@ def test_alone_and_in_a_batch(cdx, torch_cuda, rows, cols, batch, ccd):
     g = torch.Generator(device="cuda").manual_seed(rows + 3 * cols)
     inten = torch.poisson(torch.rand(rows, cols, device="cuda", generator=g) ** 8 * 6, generator=g)
     psi0 = torch.polar(inten.sqrt(), 6.28 * torch.rand(rows, cols, device="cuda", generator=g)).contiguous()
+    torch.cuda.synchronize()   # the contexts read these on streams of their own
     kw = dict(sim_ccd_bit=1, noise_level=4, exposure=0.1) if ccd else {}
     out = []
     for b in (1, batch):

@@ -27,10 +27,12 @@ def test_final_psi_from_tiles(cdx, torch_cuda, rows, cols):
     """A run's closing transform reads the iteration's narrow tiles: Psi equals the transform of the object."""
     torch = torch_cuda
     g = torch.Generator(device="cuda").manual_seed(7)
-    inten = torch.rand(rows, cols, device="cuda", generator=g)
+    inten = [torch.rand(rows, cols, device="cuda", generator=g)]
+    inten.append(inten[0] * 2)
+    torch.cuda.synchronize()   # the context reads them on a stream of its own
     with cdx.Context(cdx.default_params(rows, cols, batch=2, beta=0.9)) as ctx:
         for k in range(2):
-            ctx.set_pattern(k, (inten * (k + 1)).contiguous())
+            ctx.set_pattern(k, inten[k])
         ctx.random_start(3)
         ctx.run("2*ER")
         for k in range(2):
