@@ -164,7 +164,7 @@ int cdx_group_run(cdx_group* g, const char* algorithm, double* gpu_ms);
 /* Branch order of the group's graph: 0 (default) the contexts one after
  * another, nonzero side by side.  Each size's pass kernels already fill the GPU
  * from 192^2 x 100 up, and side-by-side branches then slow one another (the
- * 512-pattern uneven batch: 648 ms side by side, 620 ms one after another);
+ * 512-pattern uneven batch: 651 ms side by side, 535 ms one after another);
  * batches too small to fill the GPU gain from running side by side.  The next
  * cdx_group_run captures the graph again. */
 int cdx_group_set_concurrent(cdx_group* g, int concurrent);
