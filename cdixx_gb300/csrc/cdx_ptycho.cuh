@@ -108,12 +108,10 @@ __device__ __forceinline__ long long pty_tiled(int r, int c, int rows, int tl) {
 
 // Row kernels stage the CTA's object-window rows and probe rows in shared
 // memory with cp.async (pixels outside the object are zero-filled), line stride
-// N + 8 so the lines a warp reads together fall on different bank halves.  What
-// the launch before does not write is loaded ahead of the wait for it: the scan
-// index and window always (the sweep counter and the windows change between
-// sweeps), the probe from the second position of a sweep on, the pattern, and in
-// the update pass the window too (the column pass is in between).  A position
-// chain of three kernels is latency (512^2 probe, 8 positions: 0.186 -> 0.171 ms per sweep).
+// N + 8 so the lines a warp reads together fall on different bank halves.  Nothing
+// is read ahead of the wait for the launch before: the sweep's own kernels write the
+// object, the probe, the sweep counter and the windows, and a grid is promised the
+// writes of the grids before it only after its own wait.
 template <int N>
 struct PtyRow {
   static constexpr int SN = N + 8;
@@ -171,10 +169,9 @@ __global__ void __launch_bounds__(FGeom<N>::T, PtyRow<N>::MINB) pty_fwd_rk(PtyAr
   const int row0 = blockIdx.x * L;
   const int nrows = min(L, a.rows - row0);
   const int cb = row_cb_pick(a.tl, rfft_cb_max<N>());
-  const int2 w = a.win[a.order[*a.iter * a.nscan + a.k]];
-  if (a.k > 0) pty_stage_probe<N>(a, p_s, row0, nrows);
   pdl_wait_and_release();
-  if (a.k == 0) pty_stage_probe<N>(a, p_s, row0, nrows);   // the first position follows the probe's own kernels
+  const int2 w = a.win[a.order[*a.iter * a.nscan + a.k]];
+  pty_stage_probe<N>(a, p_s, row0, nrows);
   pty_stage_window<N>(a, o_s, row0, nrows, w);
   cp_commit();
   cp_wait<0>();
@@ -216,15 +213,26 @@ __global__ void __launch_bounds__(FGeom<N>::T, RGeom<FGeom<N>>::MINB_COL) pty_co
   const long long tile = (long long)blockIdx.x * N * L;
   float* int_s = reinterpret_cast<float*>(smem + L * G::LD);
   float* bs_s = int_s + L * N;
-  const int si = a.order[*a.iter * a.nscan + a.k];
-  const float* pat = a.pats + si * a.pat_stride + tile;
   const bool has_bs = a.bs != nullptr;
-  // the pattern tile (and the beamstop tile): contiguous L*N floats, bulk copies
   __shared__ uint64_t stage_bar;
   if constexpr (bulk_staging<N>()) {
-    constexpr unsigned bytes = L * N * (unsigned)sizeof(float);
     if (threadIdx.x == 0) bulk_bar_init(&stage_bar);
     __syncthreads();
+  }
+  pdl_wait_and_release();
+  const float* pat = a.pats + a.order[*a.iter * a.nscan + a.k] * a.pat_stride + tile;
+  float2 v0[F0::B][F0::R];
+#pragma unroll
+  for (int b = 0; b < F0::B; ++b) {
+    int l, j;
+    if (!bfly_of<G, F0::R>(b, 0, l, j)) continue;
+#pragma unroll
+    for (int r = 0; r < F0::R; ++r) v0[b][r] = __ldcg(a.W + tile + (long long)(j + r * F0::NR) * L + l);
+  }
+  // the pattern tile (and the beamstop tile): contiguous L*N floats, bulk copies, which
+  // land during the forward transform
+  if constexpr (bulk_staging<N>()) {
+    constexpr unsigned bytes = L * N * (unsigned)sizeof(float);
     if (threadIdx.x == 0) {
       bulk_expect(&stage_bar, bytes * (has_bs ? 2u : 1u));
       bulk_g2s(int_s, pat, bytes, &stage_bar);
@@ -237,15 +245,6 @@ __global__ void __launch_bounds__(FGeom<N>::T, RGeom<FGeom<N>>::MINB_COL) pty_co
       if (has_bs) cp_async16(bs_s + 4 * q, a.bs + tile + 4 * q, true);
     }
     cp_commit();
-  }
-  pdl_wait_and_release();
-  float2 v0[F0::B][F0::R];
-#pragma unroll
-  for (int b = 0; b < F0::B; ++b) {
-    int l, j;
-    if (!bfly_of<G, F0::R>(b, 0, l, j)) continue;
-#pragma unroll
-    for (int r = 0; r < F0::R; ++r) v0[b][r] = __ldcg(a.W + tile + (long long)(j + r * F0::NR) * L + l);
   }
   float2 v[FL::B][FL::R];
   rfft<G, 0, false>(v0, v, smem, a.tw, 0);
@@ -291,12 +290,9 @@ __global__ void __launch_bounds__(FGeom<N>::T, PtyRow<N>::MINB) pty_upd_rk(PtyAr
   const int row0 = blockIdx.x * L;
   const int nrows = min(L, a.rows - row0);
   const int cb = row_cb_pick(a.tl, rfft_cb_max<N>());
-  const int2 w = a.win[a.order[*a.iter * a.nscan + a.k]];
   const long long OC = a.obj_cols;
-  pty_stage_probe<N>(a, p_s, row0, nrows);   // land during the inverse FFT
-  pty_stage_window<N>(a, o_s, row0, nrows, w);
-  cp_commit();
   pdl_wait_and_release();
+  const int2 w = a.win[a.order[*a.iter * a.nscan + a.k]];
   float2 v0[F0::B][F0::R];
 #pragma unroll
   for (int b = 0; b < F0::B; ++b) {
@@ -306,6 +302,9 @@ __global__ void __launch_bounds__(FGeom<N>::T, PtyRow<N>::MINB) pty_upd_rk(PtyAr
     for (int r = 0; r < F0::R; ++r)
       v0[b][r] = l < nrows ? __ldcg(a.W + pty_tiled(row0 + l, j + r * F0::NR, a.rows, a.tl)) : make_float2(0.f, 0.f);
   }
+  pty_stage_probe<N>(a, p_s, row0, nrows);   // land during the inverse FFT
+  pty_stage_window<N>(a, o_s, row0, nrows, w);
+  cp_commit();
   float2 v[FL::B][FL::R];
   rfft<G, 0, true, LD>(v0, v, smem, a.tw, cb);
   cp_wait<0>();
