@@ -130,10 +130,10 @@ __device__ __forceinline__ double block_sum_d(double v, double* red) {
 // kernel of the stream be scheduled (griddepcontrol.launch_dependents; it
 // starts once every CTA of this grid has done so or exited).  The next
 // kernel's CTAs thus fill the SMs this grid's last wave leaves idle and wait
-// there, instead of being launched after it drains.  What the immediate
-// predecessor does not write is staged before the wait: when a CTA gets that far
-// every CTA of the predecessor has passed its own wait (or, a kernel without one,
-// has ended), so everything launched before the predecessor is complete.
+// there, instead of being launched after it drains.  Writes of earlier grids, the
+// ones before the predecessor too, are promised to a grid only after its own wait:
+// ahead of it a kernel reads what was complete when the host enqueued the work, and
+// nothing that a kernel of the same run writes.
 __device__ __forceinline__ void pdl_wait_and_release() {
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");

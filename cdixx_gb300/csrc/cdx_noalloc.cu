@@ -236,6 +236,7 @@ extern "C" int cdx_iterate_noalloc(int rows, int cols, int algo, float beta, int
     c.out_tiled = 1;
     c.out_stride = wst;
     c.amp = amp_t;
+    c.aux_late = 1;
     c.aux_stride = wst;
     c.tw = tw_r;
     c.cols = cols;

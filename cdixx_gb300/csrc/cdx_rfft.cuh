@@ -313,14 +313,17 @@ __global__ void __launch_bounds__(G::T, RGeom<G>::MINB_COL) col_pass_rk(ColArgs 
   float* bs_s = int_s + L * N;
   const long long aux = (long long)blockIdx.y * a.aux_stride + tile;
   // the tile's sqrt(I) (and I, beamstop for PROJ_CCD): contiguous runs of L*N
-  // floats, one bulk copy each, started before the wait for the row pass (which
-  // does not write them) and landing during the forward transform
+  // floats, one bulk copy each, landing during the forward transform.  They start
+  // before the wait for the row pass unless launches of the same call wrote the arrays
+  // (a.aux_late): a context's patterns were complete when the host enqueued the run.
   __shared__ uint64_t stage_bar;
-  if constexpr (iter) {
+  if constexpr (iter && bulk_staging<N>()) {
+    if (threadIdx.x == 0) bulk_bar_init(&stage_bar);
+    __syncthreads();
+  }
+  auto stage = [&]() {
     if constexpr (bulk_staging<N>()) {
       constexpr unsigned bytes = L * N * (unsigned)sizeof(float);
-      if (threadIdx.x == 0) bulk_bar_init(&stage_bar);
-      __syncthreads();
       if (threadIdx.x == 0) {
         const bool two = PROJ == PROJ_CCD, three = PROJ == PROJ_CCD && a.bs != nullptr;
         bulk_expect(&stage_bar, bytes * (1u + (two ? 1u : 0u) + (three ? 1u : 0u)));
@@ -339,19 +342,21 @@ __global__ void __launch_bounds__(G::T, RGeom<G>::MINB_COL) col_pass_rk(ColArgs 
       }
       cp_commit();
     }
-  }
+  };
+  if constexpr (iter) if (!a.aux_late) stage();
   pdl_wait_and_release();
   if (a.state) {
     const int f = a.state[blockIdx.y].flags;
     if (f & 6) {
       if ((f & 4) == 0 && threadIdx.x == 0) atomicOr(&a.state[blockIdx.y].flags, 4);
-      if constexpr (iter) {   // the copies land before the CTA ends
+      if constexpr (iter) if (!a.aux_late) {   // the copies land before the CTA ends
         if constexpr (bulk_staging<N>()) bulk_wait(&stage_bar, a.err);
         else cp_wait<0>();
       }
       return;
     }
   }
+  if constexpr (iter) if (a.aux_late) stage();
   const float2* in = a.in + (long long)blockIdx.y * a.in_stride;
   const bool in_t = a.in_tiled != 0;
   auto gload = [&](int l, int m) -> float2 {
@@ -563,26 +568,12 @@ __device__ __forceinline__ void row_pass_body(const RowArgs& a) {
       }
     }
   };
-  if constexpr (iter) {
-    if constexpr (!rho_in_buf) stage_rho();
-    // rows copied in late: start them towards L2 now
-    if constexpr (rho_in_buf) if (threadIdx.x < nrows) bulk_prefetch_l2(rho + (long long)threadIdx.x * N, N * (unsigned)sizeof(float2));
-    const uint32_t* mask = a.mask + (long long)blockIdx.y * a.mask_stride + (long long)row0 * WPR;
-    for (int w = threadIdx.x; w < L * WPR; w += T) {
-      const bool ok = w / WPR < nrows;
-      cp_async4(mask_s + mask_slot(w), ok ? mask + w : mask, ok);
-    }
-    cp_commit();
-  }
-  // support words and rho were last written before the column pass: only W has to be waited for
+  // rho and the support words are the run's own data: no value of them is read before the
+  // wait.  Rows copied in late start towards L2 ahead of it.
+  if constexpr (iter && rho_in_buf)
+    if (threadIdx.x < nrows) bulk_prefetch_l2(rho + (long long)threadIdx.x * N, N * (unsigned)sizeof(float2));
   pdl_wait_and_release();
-  if (a.state && (a.state[blockIdx.y].flags & 4)) {   // frozen pattern: the copies land, nothing is computed
-    if constexpr (iter) {
-      cp_wait<0>();
-      if constexpr (bulk_rho && !rho_in_buf) bulk_wait(&rho_bar, a.err);
-    }
-    return;
-  }
+  if (a.state && (a.state[blockIdx.y].flags & 4)) return;   // frozen pattern
   const float2* in = a.in + (long long)blockIdx.y * a.in_stride;
   const long long R = a.rows;
   auto goff = [&](bool t, int l, int c) -> long long {
@@ -608,6 +599,15 @@ __device__ __forceinline__ void row_pass_body(const RowArgs& a) {
         for (int r = 0; r < F0::R; ++r)
           v0[b][r] = l < nrows ? __ldcg(in + goff(a.in_tiled, l, j + r * F0::NR)) : make_float2(0.f, 0.f);
       }
+    }
+    if constexpr (iter) {   // behind the loads of W
+      if constexpr (!rho_in_buf) stage_rho();
+      const uint32_t* mask = a.mask + (long long)blockIdx.y * a.mask_stride + (long long)row0 * WPR;
+      for (int w = threadIdx.x; w < L * WPR; w += T) {
+        const bool ok = w / WPR < nrows;
+        cp_async4(mask_s + mask_slot(w), ok ? mask + w : mask, ok);
+      }
+      cp_commit();
     }
     if constexpr (iter && rho_in_buf) {
       rfft<G, 0, true, LD>(v0, v, buf, tw, cb, [&]() {

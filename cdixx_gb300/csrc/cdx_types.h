@@ -99,6 +99,7 @@ struct ColArgs {
   int pdl_mode;            // as RowArgs::pdl_mode
   int* err;                // as RowArgs::err
   int thin;                // as RowArgs::thin; column-tiled arrays then have that geometry's width
+  int aux_late;            // 1: launches of the same call wrote amp, inten or bs, so they are read after the wait for the predecessor
 };
 
 // Launch helpers exported by the per-size translation units.
