@@ -627,9 +627,10 @@ __device__ __forceinline__ void fft_pass_umma16(float2* buf, const float2* tw, U
     }
     umma::mma_commit(U.bar);
   }
-  if (!umma::mbar_wait(U.bar, U.phase) && (t & 31) == 0 && U.err) atomicOr(U.err, 1);
+  if (!umma::warp_wait(U.bar, U.phase) && (t & 31) == 0 && U.err) atomicOr(U.err, 1);
   U.phase ^= 1u;
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  __syncwarp();
   uint32_t v[32];
   {
     const unsigned ta = U.tmem + ((unsigned)((warp & 3) * 32) << 16) + (unsigned)((warp >> 2) * 32);

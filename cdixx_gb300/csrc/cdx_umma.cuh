@@ -130,6 +130,15 @@ __device__ __forceinline__ bool mbar_wait_or_abort(unsigned bar, unsigned parity
   return false;
 }
 
+// The waits for a whole warp: one result for all its lanes, which are together again when
+// they have it, as tcgen05.ld and the other .aligned instructions need them.
+__device__ __forceinline__ bool warp_wait(unsigned bar, unsigned parity) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity));
+}
+__device__ __forceinline__ bool warp_wait_or_abort(unsigned bar, unsigned parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait_or_abort(bar, parity, abort_flag));
+}
+
 template <int BN, class Op>
 __global__ void __launch_bounds__(PS_THREADS, 1) k_umma_ps(Op op, int M, int N, int K, int* __restrict__ err) {
   static_assert(BN == 32 || BN == 64 || BN == 128, "UMMA N tile");
@@ -218,7 +227,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) k_umma_ps(Op op, int M, int N, 
     cp_wait<0>();
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     if (failed) {
-      if ((tid & 31) == 0) give_up();
+      give_up();
     } else {
       for (long long q = g > WS_D ? g - WS_D : 0; q < g; ++q) mbar_arrive(smem_u32(&full[q % WS_ST]));
     }
@@ -228,7 +237,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) k_umma_ps(Op op, int M, int N, 
     int t = 0;
     for (int tile = blockIdx.x; tile < MT; tile += gridDim.x, ++t) {
       const int b = t & 1;
-      if (!mbar_wait_or_abort(smem_u32(&tfull[b]), (unsigned)((t >> 1) & 1), &abort_flag)) {
+      if (!warp_wait_or_abort(smem_u32(&tfull[b]), (unsigned)((t >> 1) & 1), &abort_flag)) {
         if (lane == 0) give_up();
         break;
       }
@@ -238,6 +247,7 @@ __global__ void __launch_bounds__(PS_THREADS, 1) k_umma_ps(Op op, int M, int N, 
       for (int c0 = 0; c0 < BN; c0 += 16) {
         uint32_t v[16];
         const unsigned ta = tmem + ((unsigned)(ew * 32) << 16) + (unsigned)(b * BN + c0);
+        __syncwarp();   // lanes without a row or columns to store skip that
         asm volatile(
             "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
             : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
@@ -294,8 +304,9 @@ __global__ void __launch_bounds__(PS_THREADS, 1) k_umma_ps(Op op, int M, int N, 
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   if (warp == 8) {
-    if (!mbar_wait(smem_u32(&done), 0) && (tid & 31) == 0) atomicExch(err, 1);
+    if (!warp_wait(smem_u32(&done), 0) && (tid & 31) == 0) atomicExch(err, 1);
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TC) : "memory");
   }
 }

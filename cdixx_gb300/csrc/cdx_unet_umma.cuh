@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(kCuThreads, 3) k_conv_umma(const __grid_consta
     cp_wait<0>();
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     if (failed) {
-      if (lane == 0) give_up();
+      give_up();
     } else if (D == 1 && g > 0) {
       mbar_arrive(smem_u32(&afull[(g - 1) % a.npatch]));
     }
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(kCuThreads, 3) k_conv_umma(const __grid_consta
       const int gy = r / tx * kCuTH + ew * 4, gx = (r % tx) * kCuTW + (lane >> 2);
       for (int cls = 0; cls < a.ncls; ++cls, ++q) {
         const int b = q & 1;
-        if (!mbar_wait_or_abort(smem_u32(&tfull[b]), (unsigned)((q >> 1) & 1), &abort_flag)) {
+        if (!warp_wait_or_abort(smem_u32(&tfull[b]), (unsigned)((q >> 1) & 1), &abort_flag)) {
           if (lane == 0) give_up();
           failed = true;
           break;
@@ -182,6 +182,7 @@ __global__ void __launch_bounds__(kCuThreads, 3) k_conv_umma(const __grid_consta
         for (int c0 = 0; c0 < N; c0 += 16) {
           uint32_t v[16];
           const unsigned ta = tmem + ((unsigned)(ew * 32) << 16) + (unsigned)(b * N + c0);
+          __syncwarp();   // the previous channels have been read, by lanes outside the grid too
           asm volatile(
               "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
@@ -189,7 +190,6 @@ __global__ void __launch_bounds__(kCuThreads, 3) k_conv_umma(const __grid_consta
               : "r"(ta)
               : "memory");
           asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-          __syncwarp();   // the previous channels have been read
 #pragma unroll
           for (int k = 0; k < 4; ++k)
             *reinterpret_cast<uint4*>(tr + lane * kCuEpi + 4 * k) = make_uint4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
@@ -317,8 +317,9 @@ __global__ void __launch_bounds__(kCuThreads, 3) k_conv_umma(const __grid_consta
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   if (warp == 8) {
-    if (!mbar_wait(smem_u32(&done), 0) && lane == 0) atomicExch(err, 1);
+    if (!warp_wait(smem_u32(&done), 0) && lane == 0) atomicExch(err, 1);
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(cols) : "memory");
   }
 }
@@ -540,12 +541,12 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_wgrad_umma(const __grid_const
     umma::cp_wait<0>();
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     if (failed) {
-      if (lane == 0) give_up();
+      give_up();
     } else {
       for (int q = g > kWgAhead ? g - kWgAhead : 0; q < g; ++q) mbar_arrive(smem_u32(&full[q % kWgStages]));
     }
     // ------------------------------------------------------------ partial sums
-    if (!mbar_wait_or_abort(smem_u32(&done), 0, &abort_flag) || abort_flag) {
+    if (!__all_sync(0xffffffffu, mbar_wait_or_abort(smem_u32(&done), 0, &abort_flag) && !abort_flag)) {
       if (lane == 0) give_up();
     } else {
       asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
@@ -555,6 +556,7 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_wgrad_umma(const __grid_const
         for (int c0 = 0; c0 < ncol; c0 += 16) {
           uint32_t v[16];
           const unsigned ta = tmem + ((unsigned)(warp * 32) << 16) + (unsigned)(t * ncol + c0);
+          __syncwarp();   // lanes past the channels skip the stores
           asm volatile(
               "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
@@ -614,8 +616,9 @@ __global__ void __launch_bounds__(kWgThreads, 1) k_wgrad_umma(const __grid_const
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   if (warp == 4) {
-    if (!mbar_wait(smem_u32(&done), 0) && lane == 0) atomicExch(err, 1);
+    if (!warp_wait(smem_u32(&done), 0) && lane == 0) atomicExch(err, 1);
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(cols) : "memory");
   }
 }
