@@ -1100,6 +1100,10 @@ int cdx_unet_create(const cdx_unet_config* c, void* stream, cdx_unet** out) {
   if (c->groups < 1 || c->base % c->groups || (kThreads % (c->base / c->groups)) ||
       c->base / c->groups > kThreads)
     return set_error(CDX_ERR_ARG, "groups must divide base (and base/groups divide 256)");
+  // the statistics kernels give each of a group's channels a thread of 256 (channels double per level)
+  if (((long long)(c->base / c->groups) << (c->levels - 1)) > kThreads)
+    return set_error(CDX_ERR_ARG, "a group may hold at most 256 channels at the deepest level "
+                                  "(base/groups * 2^(levels-1))");
   if (c->n < 16 || c->n % (8 << (c->levels - 1))) return set_error(CDX_ERR_SIZE, "n must be a multiple of 8*2^(levels-1)");
   if (c->batch < 1) return set_error(CDX_ERR_ARG, "batch must be >= 1");
   if (!cdx_size_supported(c->n)) return set_error(CDX_ERR_SIZE, "n is not a supported FFT length");

@@ -38,7 +38,7 @@ typedef struct {
   int levels;         /* resolutions (>= 2) */
   int base;           /* channels at full resolution (a multiple of 8) */
   int batch;          /* largest batch a call may pass */
-  int groups;         /* GroupNorm groups (divides base) */
+  int groups;         /* GroupNorm groups (divides base; at most 256 channels a group at the deepest level) */
   float slope;        /* LeakyReLU negative slope */
   float support_weight; /* w_s */
   unsigned long long seed; /* weight initialisation */
