@@ -675,7 +675,7 @@ struct Net {
   unsigned* mx = nullptr;  // largest log(1 + I) per pattern, float bits
   int* twin = nullptr;
   float2* wrk = nullptr;   // warm start scratch
-  int* umma_err = nullptr; // set by a tcgen05 tile whose pipeline wait timed out
+  int* umma_err = nullptr; // set by a tcgen05 tile whose pipeline wait timed out (check_umma)
   int adam_t = 0;
   bool dep = false;        // launch the forward's kernels dependently (small passes)
   bool weights_dirty = true;
@@ -1180,11 +1180,15 @@ int cdx_unet_get_grads(const cdx_unet* u, float* host, long long count) {
   return CDX_OK;
 }
 
+// A wait that ran out in this call's kernels is reported here and cleared for the next call's.
 static int check_umma(Net* n) {
   int flag = 0;
   U_CK(cudaMemcpyAsync(&flag, n->umma_err, sizeof(int), cudaMemcpyDeviceToHost, n->st));
   U_CK(cudaStreamSynchronize(n->st));
-  if (flag) return set_error(CDX_ERR_CUDA, "tensor-core GEMM pipeline wait timed out");
+  if (flag) {
+    U_CK(cudaMemsetAsync(n->umma_err, 0, sizeof(int), n->st));
+    return set_error(CDX_ERR_CUDA, "tensor-core GEMM pipeline wait timed out");
+  }
   return CDX_OK;
 }
 
