@@ -265,6 +265,11 @@ void plan_shrinkwrap(const cdx_ctx* c, int count, SwPlan& P) {
   }
 }
 
+// Whether patterns of a run may stop before its end.
+bool may_stop(const cdx_ctx* c) {
+  return c->p.rf_every > 0 && (c->p.stop_rfactor > 0 || c->p.plateau_iters > 0 || c->own_stops);
+}
+
 // One pass of the iteration over the patterns [p0, p0 + nb).
 int col_iter(cdx_ctx* c, int p0, int nb, bool from_psi, bool rf, float2* psi_proj = nullptr) {
   ColArgs a{};
@@ -297,6 +302,7 @@ int col_iter(cdx_ctx* c, int p0, int nb, bool from_psi, bool rf, float2* psi_pro
   a.pdl_mode = c->tune_pdl_col;
   a.err = c->derr;
   a.thin = c->thin;
+  a.may_stop = may_stop(c);
   CDX_CK(col_launcher(c->rows)(a, nb, c->st));
   return CDX_OK;
 }
@@ -324,6 +330,7 @@ int row_iter(cdx_ctx* c, int p0, int nb, int algo) {
   a.pdl_mode = c->tune_pdl_row;
   a.err = c->derr;
   a.thin = c->thin;
+  a.may_stop = may_stop(c);
   CDX_CK(row_launcher(c->cols)(a, nb, c->st));
   return CDX_OK;
 }
@@ -393,8 +400,7 @@ int enqueue_run(cdx_ctx* c, const std::vector<int>& steps, const SwPlan& sw, boo
   const bool prtf = c->pr_map && c->p.prtf_iter >= 0;
   c->pr_reached = false;
   if (prtf) CDX_CK(cudaMemsetAsync(c->pr_map, 0, sizeof(float2) * n_all, c->st));
-  const bool stops = c->p.rf_every > 0 && (c->p.stop_rfactor > 0 || c->p.plateau_iters > 0 || c->own_stops);
-  const int chunks = prtf ? 1 : chunks_of(c->npx, c->wstride, c->batch, stops);
+  const int chunks = prtf ? 1 : chunks_of(c->npx, c->wstride, c->batch, may_stop(c));
   for (size_t at = 0; at < steps.size(); ++at) {
     const int a = steps[at];
     ++step;   // phaseRetrieve's iter: every step, shrinkwraps included

@@ -63,7 +63,7 @@ struct RowArgs {
   long long out_stride;
   long long rho_stride;
   long long mask_stride;   // mask words between patterns
-  const PatState* state;   // optional: CTAs of frozen patterns (flags bit 2) return at once
+  const PatState* state;   // optional: CTAs of frozen patterns (flags bit 2) return at once, nothing copied (may_stop)
   int tc;                  // 1: radix-16 passes on the tensor cores (BF16 split, FP32 accumulate)
   float scale;             // factor applied on store (1 = none)
   float inv_n;             // 1/(rows*cols) (applyNorm after the inverse FFT)
@@ -72,6 +72,7 @@ struct RowArgs {
   int pdl_mode;            // 0: the per-length default, 1: plain launch, 2: programmatic dependent launch
   int* err;                // optional: bit 0 set when a bulk copy's wait ran out
   int thin;                // 1: the geometry for small work (lengths that have one)
+  int may_stop;            // 1: patterns of the run may freeze (state given): look at the flag before anything is fetched early
 };
 
 struct ColArgs {
@@ -100,6 +101,7 @@ struct ColArgs {
   int* err;                // as RowArgs::err
   int thin;                // as RowArgs::thin; column-tiled arrays then have that geometry's width
   int aux_late;            // 1: launches of the same call wrote amp, inten or bs, so they are read after the wait for the predecessor
+  int may_stop;            // as RowArgs::may_stop
 };
 
 // Launch helpers exported by the per-size translation units.

@@ -35,7 +35,7 @@ def test_pass_kernels_read_nothing_of_the_run_early():
     assert not re.findall(r"a\.(?:in|out|psi_out)\b", col)
     # the pattern arrays are read early where the host had them complete; the call that
     # makes them on its own stream says so
-    assert re.search(r"if \(!a\.aux_late\) stage\(\);", col)
+    assert re.search(r"early = iter && !a\.aux_late && ", col)
     assert re.search(r"c\.aux_late = 1;", (CSRC / "cdx_noalloc.cu").read_text())
 
 
