@@ -8,6 +8,7 @@
 // captured once into a CUDA graph and replayed.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -133,7 +134,7 @@ struct cdx_ctx {
   PrtfState* pr_state = nullptr;
   bool pr_valid = false;       // the last run reached prtf_iter
   bool pr_reached = false;     // set while enqueueing
-  bool own_stops = false;      // a pattern was given a stop of its own
+  std::vector<char> own_stop;  // the pattern has a stop of its own (cdx_set_stop_rfactor)
 
   // launch variant (autotune): RowArgs/ColArgs knobs, and what was measured
   int tune_pdl_col = 0, tune_pdl_row = 0, tune_cb_plus1 = 0;   // pdl: 0 per-length default, 1 plain, 2 PDL
@@ -267,7 +268,8 @@ void plan_shrinkwrap(const cdx_ctx* c, int count, SwPlan& P) {
 
 // Whether patterns of a run may stop before its end.
 bool may_stop(const cdx_ctx* c) {
-  return c->p.rf_every > 0 && (c->p.stop_rfactor > 0 || c->p.plateau_iters > 0 || c->own_stops);
+  return c->p.rf_every > 0 && (c->p.stop_rfactor > 0 || c->p.plateau_iters > 0 ||
+                               std::find(c->own_stop.begin(), c->own_stop.end(), 1) != c->own_stop.end());
 }
 
 // One pass of the iteration over the patterns [p0, p0 + nb).
@@ -784,7 +786,7 @@ int run_impl(cdx_ctx* c, const char* algorithm) {
   const bool piw = c->psi_in_work;
   if (c->p.use_graph) {
     char key[64];
-    snprintf(key, sizeof key, "|%d|%p", (int)piw, (void*)c->weights);
+    snprintf(key, sizeof key, "|%d|%d|%p", (int)piw, (int)may_stop(c), (void*)c->weights);
     std::string k = std::string(algorithm) + key;
     if (k != c->gkey || !c->gexec) {
       if (c->gexec) { cudaGraphExecDestroy(c->gexec); c->gexec = nullptr; }
@@ -842,7 +844,7 @@ int group_run_impl(cdx_group* g, const char* algorithm, double* gpu_ms) {
     int e = prepare_run(c, algorithm, steps[i], sw[i]);
     if (e) return e;
     char k[64];
-    snprintf(k, sizeof k, "|%d|%p", (int)c->psi_in_work, (void*)c->weights);
+    snprintf(k, sizeof k, "|%d|%d|%p", (int)c->psi_in_work, (int)may_stop(c), (void*)c->weights);
     key += k;
   }
   if (key != g->gkey || !g->gexec) {
@@ -976,6 +978,7 @@ int cdx_create(const cdx_params* p, void* stream, cdx_ctx** out) {
   c->wpr = (p->cols + 31) >> 5;
   c->have_pattern.assign(p->batch, 0);
   c->fresh.assign(p->batch, 0);
+  c->own_stop.assign(p->batch, 0);
   cudaGetDevice(&c->device);
   auto fail = [&](int code) { cdx_destroy(c); return code; };
   if (stream) {
@@ -1275,9 +1278,9 @@ int cdx_set_support(cdx_ctx* c, int idx, const float* support, int where) {
 
 int cdx_set_stop_rfactor(cdx_ctx* c, int idx, double stop) {
   if (!c || idx < 0 || idx >= c->batch || !(stop >= 0.0)) return set_error(CDX_ERR_ARG, "bad stop argument");
-  c->own_stops = c->own_stops || stop > 0;
   CDX_CK(cudaMemcpyAsync(&c->dstate[idx].stop, &stop, sizeof(double), cudaMemcpyHostToDevice, c->st));
   CDX_CK(cudaStreamSynchronize(c->st));
+  c->own_stop[idx] = stop > 0;
   return CDX_OK;
 }
 
@@ -1395,6 +1398,7 @@ int ctx_reset(cdx_ctx* c) {
   }
   c->have_pattern.assign(c->batch, 0);
   c->fresh.assign(c->batch, 0);
+  c->own_stop.assign(c->batch, 0);
   c->have_initial = false;
   c->psi_in_work = false;
   c->pr_valid = false;
