@@ -892,9 +892,7 @@ int group_run_impl(cdx_group* g, const char* algorithm, double* gpu_ms) {
   return CDX_OK;
 }
 
-// The statistics of the pattern whose state c->back holds.
-int stats_of_back(cdx_ctx* c, cdx_stats* s) {
-  const PatState& h = c->back->state;
+int fill_stats(cdx_ctx* c, const PatState& h, cdx_stats* s) {
   memset(s, 0, sizeof *s);
   s->steps = c->last_steps;
   s->iterations = c->last_iters;
@@ -910,13 +908,6 @@ int stats_of_back(cdx_ctx* c, cdx_stats* s) {
   if (cudaEventElapsedTime(&ms, c->ev0, c->ev1) == cudaSuccess) s->gpu_ms = ms;
   else cudaGetLastError();
   return CDX_OK;
-}
-
-int fill_stats(cdx_ctx* c, int idx, cdx_stats* s) {
-  if (!s) return CDX_OK;
-  CDX_CK(cudaMemcpyAsync(&c->back->state, c->dstate + idx, sizeof(PatState), cudaMemcpyDeviceToHost, c->st));
-  CDX_CK(cudaStreamSynchronize(c->st));
-  return stats_of_back(c, s);
 }
 
 }  // namespace
@@ -1346,12 +1337,16 @@ int cdx_run(cdx_ctx* c, const char* algorithm, cdx_stats* stats) {
     CDX_CK(cudaMemset(c->derr, 0, sizeof(int)));
     return set_error(CDX_ERR_CUDA, "a pass kernel's bulk staging copy timed out; the run's results are invalid");
   }
-  return stats ? stats_of_back(c, stats) : CDX_OK;
+  return stats ? fill_stats(c, c->back->state, stats) : CDX_OK;
 }
 
 int cdx_get_stats(cdx_ctx* c, int idx, cdx_stats* s) {
   if (!c || idx < 0 || idx >= c->batch) return set_error(CDX_ERR_ARG, "bad stats argument");
-  return fill_stats(c, idx, s);
+  if (!s) return CDX_OK;
+  PatState h;   // the caller's own: several threads may ask at once
+  CDX_CK(cudaMemcpyAsync(&h, c->dstate + idx, sizeof h, cudaMemcpyDeviceToHost, c->st));
+  CDX_CK(cudaStreamSynchronize(c->st));
+  return fill_stats(c, h, s);
 }
 
 int cdx_get_object(cdx_ctx* c, int idx, float* out, int where) {
