@@ -956,7 +956,7 @@ def run_case(argv):
     c.add_argument("--steps", type=int, default=3)
     c.add_argument("--levels", type=int, default=4)
     c.add_argument("--base", type=int, default=32)
-    c.add_argument("--umma", type=int, default=0, help="1: tcgen05 convolutions, 0: mma.sync")
+    c.add_argument("--umma", type=int, default=0, help="kernels of the convolutions (cdx_unet_config::umma)")
     c = sub.add_parser("ptycho")
     c.add_argument("--probe", type=int, default=512)
     c.add_argument("--object", type=int, default=1280)

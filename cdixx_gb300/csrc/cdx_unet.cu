@@ -879,6 +879,9 @@ bool plan_umma(const GemmArgs& g, const __nv_bfloat16* packed, ConvUmma& a, int&
   return cu_plan(a, s.KH * s.KW, smem);
 }
 
+// cdx_unet_config::umma 2 and 3: every convolution and weight gradient on the gathering kernels
+bool gather_all(const Net* u) { return u->cfg.umma == 2 || u->cfg.umma == 3; }
+
 // forward (DGRAD false) or data-gradient GEMM: k_conv_umma where the layer fits it (`packed`:
 // its weights); else the gathering kernels, tcgen05 when the net is configured for them
 template <bool DGRAD>
@@ -886,14 +889,14 @@ int launch_gemm(const Net* u, const GemmArgs& a, const __nv_bfloat16* packed, cu
   const ConvShape& s = a.s;
   ConvUmma c;
   int smem = 0;
-  if (plan_umma<DGRAD>(a, packed, c, smem)) {
+  if (!gather_all(u) && plan_umma<DGRAD>(a, packed, c, smem)) {
     U_CK(launch_conv_umma(c, smem, u->umma_err, u->dep, st));
     return CDX_OK;
   }
   const long long M = DGRAD ? (long long)s.N * s.H * s.W : (long long)s.N * s.Ho * s.Wo;
   const int NC = DGRAD ? s.Cin : s.Cout;
   const int K = DGRAD ? s.KH * s.KW * s.Cout : s.KH * s.KW * s.Cin;
-  if (u->cfg.umma) {
+  if (u->cfg.umma != 0 && u->cfg.umma != 2) {
     using Op = typename std::conditional<DGRAD, ConvDgradOp, ConvFwdOp>::type;
     const Op op{a};
     if (NC <= 32) return launch_umma<32>(op, M, NC, K, u->umma_err, st);
@@ -925,7 +928,7 @@ int launch_wgrad(Net* u, GemmArgs a, const Layer& l) {
   w.KH = s.KH; w.KW = s.KW; w.S = s.S; w.P = s.P;
   w.M = (int)M;
   w.m_per_split = (int)mps;
-  if (wg_plan(w, (int)splits, sm_count())) U_CK(launch_wgrad_umma(w, (int)splits, u->umma_err, u->st));
+  if (!gather_all(u) && wg_plan(w, (int)splits, sm_count())) U_CK(launch_wgrad_umma(w, (int)splits, u->umma_err, u->st));
   else k_conv_wgrad<<<dim3(tx, ty, (unsigned)splits), 128, 0, u->st>>>(a);
   const long long tot = (long long)l.wco_r * l.k * l.k * l.wci_r;
   k_wgrad_reduce<<<grid_for(tot), kThreads, 0, u->st>>>(u->wpart, (int)splits, l.wco_r, l.wci_r, l.wco_p, l.wci_p,

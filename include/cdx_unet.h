@@ -44,8 +44,9 @@ typedef struct {
   unsigned long long seed; /* weight initialisation */
   int umma;           /* kernels of the forward and data-gradient convolutions whose channels do not fit the
                          tcgen05 patch kernel (16 to 256, whole 16s; those always take it): 1 tcgen05 with
-                         gathered tiles, 0 (default) warp-level mma.sync.  The weight gradient is tcgen05 where a row holds whole 16s of pixels.
-                         All of them give the same bits */
+                         gathered tiles, 0 (default) warp-level mma.sync.  The weight gradient is tcgen05 where a
+                         row holds whole 16s of pixels.  3 and 2: as 1 and 0 for every layer, the weight gradient on
+                         mma.sync, to compare with.  All of them give the same bits */
 } cdx_unet_config;
 
 int cdx_unet_config_default(cdx_unet_config* c);
