@@ -40,3 +40,10 @@ def test_final_psi_from_tiles(cdx, torch_cuda, rows, cols):
             psi = torch.from_numpy(ctx.get_fourier(k)).cuda()
             ref = torch.fft.fft2(rho)
             assert float((psi - ref).norm() / ref.norm()) < 5e-7
+
+
+@pytest.mark.parametrize("rows,cols,batch", [(1024, 1024, 3), (1024, 16, 129), (1024, 24, 90), (1024, 2048, 2)])
+def test_wide_columns_of_1024_match_float64(cdx, torch_cuda, rows, cols, batch):
+    """From 2^21 pixels on, below which lengths of 1024 take the geometry for small work: row-major input."""
+    assert rows * cols * batch > 1 << 21 and (cols + 7) // 8 * batch >= 152
+    test_wide_columns_match_float64(cdx, torch_cuda, rows, cols, batch)
