@@ -875,6 +875,11 @@ int group_run_impl(cdx_group* g, const char* algorithm, double* gpu_ms) {
     if (ce != cudaSuccess) return set_error(CDX_ERR_CUDA, std::string("group instantiate: ") + cudaGetErrorString(ce));
     g->gkey = key;
   }
+  // after what the contexts' own streams hold (a cdx_run_async that is still running, say)
+  for (size_t i = 0; i < n; ++i) {
+    CDX_CK(cudaEventRecord(g->joins[i], g->ctxs[i]->st));
+    CDX_CK(cudaStreamWaitEvent(g->st, g->joins[i], 0));
+  }
   CDX_CK(cudaEventRecord(g->ev0, g->st));
   CDX_CK(cudaGraphLaunch(g->gexec, g->st));
   CDX_CK(cudaEventRecord(g->ev1, g->st));

@@ -158,7 +158,7 @@ int cdx_get_stats(cdx_ctx* ctx, int idx, cdx_stats* stats);
  * and stay alive while the group exists. */
 typedef struct cdx_group cdx_group;
 int cdx_group_create(cdx_ctx* const* ctxs, int n, cdx_group** out);
-/* Runs `algorithm` on every context; synchronises; *gpu_ms gets the graph's
+/* Runs `algorithm` on every context, after the work on their streams; synchronises; *gpu_ms gets the graph's
  * device time (may be NULL).  Per-pattern results: cdx_get_stats / cdx_get_*. */
 int cdx_group_run(cdx_group* g, const char* algorithm, double* gpu_ms);
 /* Branch order of the group's graph: 0 (default) the contexts one after
