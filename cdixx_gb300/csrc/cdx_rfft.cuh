@@ -78,8 +78,9 @@ __device__ __forceinline__ bool bfly_of(int b, int cb, int& l, int& j) {
 // 16 / lines columns in all, so lines 16 / lines mod 16 apart put them on 16
 // different bank pairs; from cb = 4 on a half-warp stays on one line and the
 // column pass's stride (16 / L mod 16 for its line-fastest map) serves both.
-// Only 48 to 192 and 384 get a stride of their own (192^2 x96: 60.9 -> 46.8 us
-// per iteration, 384^2 x32: 60.8 -> 56.0).
+// 32, 64, 96, 128 and 384 get a stride of their own; at 48 and 192 the rule gives the
+// column pass's (384^2 x32: 60.8 -> 56.0 us per iteration; 192^2 x96 on the 16 lines that
+// 256 threads hold 60.9 -> 46.8).
 template <class G>
 __host__ __device__ constexpr int row_line_stride() {
   constexpr int cb = row_cb_pick(G::LOG2L, rfft_cb_max<G::N>());
@@ -491,8 +492,8 @@ __global__ void __launch_bounds__(G::T, RGeom<G>::MINB_COL) col_pass_rk(ColArgs 
 // are one base address plus whole-tile strides, with no per-element index
 // arithmetic.  The launcher takes the general kernel otherwise.
 // The compile-time layout needs every pass's element stride to be whole tiles:
-// 2^log2(L) divides N/R for each radix R (true from 256 up; at 16..192 the
-// column tiles are wider than that).
+// 2^log2(L) divides N/R for each radix R (true from 128 up, and from 256 up with the
+// wider tiles of Geom; below, the column tiles are wider than that).
 template <class G>
 __host__ __device__ constexpr bool row_sq_ok_g() { return G::LOG2L <= rfft_cb_max<G::N>(); }
 template <int N>
