@@ -844,7 +844,7 @@ int group_run_impl(cdx_group* g, const char* algorithm, double* gpu_ms) {
     int e = prepare_run(c, algorithm, steps[i], sw[i]);
     if (e) return e;
     char k[64];
-    snprintf(k, sizeof k, "|%d|%d|%p", (int)c->psi_in_work, (int)may_stop(c), (void*)c->weights);
+    snprintf(k, sizeof k, "|%d|%d|%p|%p", (int)c->psi_in_work, (int)may_stop(c), (void*)c->weights, (void*)c->bs_t);
     key += k;
   }
   if (key != g->gkey || !g->gexec) {

@@ -42,3 +42,30 @@ def test_group_run_follows_asynchronous_runs(cdx, torch_cuda, concurrent):
             c.close()
     for (a, s), (b, t) in zip(*out):
         assert np.array_equal(a, b) and np.array_equal(s, t) and np.isfinite(a).all()
+
+
+@pytest.mark.gpu
+def test_group_run_takes_a_beamstop_set_after_a_run(cdx, torch_cuda):
+    """A beamstop given after the group captured the algorithm is in its next run, as in a context's."""
+    torch = torch_cuda
+    n = 128
+    g = torch.Generator(device="cuda").manual_seed(8)
+    pat = torch.poisson(torch.rand(n, n, device="cuda", generator=g) ** 8 * 6, generator=g)
+    stop = (torch.rand(n, n, device="cuda", generator=g) > 0.7).float()
+    torch.cuda.synchronize()   # the contexts read them on streams of their own
+    p = cdx.default_params(n, n, beta=0.9, sim_ccd_bit=1, noise_level=4, exposure=0.1)
+    out = []
+    for grouped in (False, True):
+        with cdx.Context(p) as ctx:
+            owner = cdx.Group([ctx]) if grouped else ctx
+            ctx.set_pattern(0, pat)
+            for given in (False, True):
+                if given:
+                    ctx.set_beamstop(0, stop)
+                ctx.random_start(3)
+                owner.run("5*RAAR")
+                out.append(ctx.get_object(0))
+            if grouped:
+                owner.close()
+    assert np.array_equal(out[0], out[2]) and np.array_equal(out[1], out[3])
+    assert not np.array_equal(out[0], out[1])
